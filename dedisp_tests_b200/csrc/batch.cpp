@@ -9,6 +9,8 @@
 #include "dedisp_b200.h"
 #include "errors.hpp"
 #include "host_math.hpp"
+#include "tdd_engine.hpp"
+#include "tdd_pattern.hpp"
 
 namespace dedisp {
 namespace detail {
@@ -36,7 +38,8 @@ struct TddBatch::Layout {
     std::vector<kern::DedisperseArgs> args;   // host copy (device pointers)
     std::vector<size_t> tr_off;               // words into the workspace
     std::vector<size_t> pitch;                // words per channel row
-    bool quad = false;                        // quad-strided rows (8-bit quad variants)
+    bool quad = false;                        // strided rows (quad variants, pattern kernel)
+    bool pattern = false;                     // shared channel-group sums (tdd_pattern.hpp)
     int period = 0;                           // quad: P words
     std::vector<size_t> q_off;                // quad: rows' offset in the workspace (words)
     std::vector<size_t> qpitch;               // quad: words per row
@@ -172,6 +175,47 @@ void TddBatch::set_beams(std::vector<BatchBeamSpec> beams)
     RT_CHECK(cudaMemcpy(m_d_perm.get(), perm.data(), perm.size() * 4, cudaMemcpyHostToDevice));
     m_beams = std::move(st);
     m_dirty = true;
+    prepare_patterns();
+}
+
+// Pattern tables of every beam; the default shape uses the pattern kernel if
+// it takes each of them and is the faster one for each.
+void TddBatch::prepare_patterns()
+{
+    m_pattern = false;
+    if (m_general_mask || m_beams.empty() || m_chan.empty()) return;
+    std::vector<float> cdl(m_chan.size());
+    for (size_t j = 0; j < cdl.size(); ++j) cdl[j] = m_delays[m_chan[j]];
+    long words = 0;
+    size_t tiles = 0;
+    const size_t bt = (size_t)kern::pattern_block_samples(m_nbits, 4);
+    for (const BeamState& t : m_beams) {
+        if (!pattern_takes(t.sorted, cdl, m_nbits)) return;
+        tiles += (t.sorted.size() + kern::kPatternDms - 1) / kern::kPatternDms * ((t.nout + bt - 1) / bt);
+    }
+    // a period at which every beam's groups fit
+    bool wide = true;
+    while (wide) {
+        m_lane_words = kern::pattern_lane_words(m_nbits, tiles, words);
+        if (!m_lane_words) return;
+        m_tables.resize(m_beams.size());
+        for (size_t b = 0; b < m_beams.size(); ++b) {
+            const BeamState& t = m_beams[b];
+            if (!m_tables[b]) m_tables[b].reset(new PatternTables());
+            m_tables[b]->size(m_d_dms.get<float>() + t.dm_off, t.sorted.size(), m_d_chan.get<int32_t>(),
+                              m_d_cdl.get<float>(), m_chan.size(), m_nchans, m_nbits, m_lane_words, nullptr);
+        }
+        wide = false;
+        for (auto& t : m_tables) {
+            const PatternTables::Fit fit = t->fit(nullptr);
+            words = std::max(words, t->group_words());
+            if (fit == PatternTables::kRowsFaster) return;
+            if (fit == PatternTables::kTooWide) wide = true;
+        }
+    }
+    for (auto& t : m_tables) t->emit(nullptr);
+    RT_CHECK(cudaStreamSynchronize(nullptr));
+    m_pattern = true;
 }
 
 void TddBatch::set_shape(const BatchShape& shape)
@@ -194,17 +238,20 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
     const int nb = m_nbits, v = shape.variant;
     const int spw = 32 / nb;
     const bool want_tiled = !m_general_mask;
-    const size_t bd = (size_t)kern::tiled_block_dms(nb, v);
-    const size_t bt = (size_t)kern::tiled_block_samples(nb, v);
+    // the default shape, sized by the library, is the pattern kernel where
+    // that is the faster one
+    L.pattern = want_tiled && m_pattern && v == kern::tiled_default_variant(nb) && shape.chan_per_stage == 0;
+    const size_t bd = L.pattern ? (size_t)kern::kPatternDms : (size_t)kern::tiled_block_dms(nb, v);
+    const size_t bt = L.pattern ? (size_t)kern::pattern_block_samples(nb, m_lane_words) : (size_t)kern::tiled_block_samples(nb, v);
     const int J = kern::tiled_lane_words(nb, v);
-    const bool quad = want_tiled && kern::tiled_variant_quad(nb, v);
+    const bool quad = want_tiled && (L.pattern || kern::tiled_variant_quad(nb, v));
     const size_t nbeams = m_beams.size();
     L.args.resize(nbeams);
     L.tr_off.resize(nbeams);
     L.pitch.resize(nbeams);
     L.q_off.assign(nbeams, 0);
     L.qpitch.assign(nbeams, 0);
-    L.period = 32 * J;
+    L.period = L.pattern ? 32 * m_lane_words : 32 * J;
     L.nbx.resize(nbeams);
     L.units.resize(nbeams);
     L.start.assign(nbeams + 1, 0);
@@ -212,7 +259,7 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
     // sends the whole batch to the plain kernel.
     std::vector<int> W(nbeams, 0), CS(nbeams, 0);
     bool tiled = want_tiled;
-    for (size_t b = 0; b < nbeams && tiled; ++b) {
+    for (size_t b = 0; b < nbeams && tiled && !L.pattern; ++b) {
         const BeamState& t = m_beams[b];
         uint32_t span = 0;
         for (size_t i = 0; i < t.sorted.size(); i += bd) {
@@ -230,6 +277,10 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
         W[b] = (int)w;
         CS[b] = shape.chan_per_stage > 0 ? std::min(shape.chan_per_stage, fit) : fit;
     }
+    if (!tiled) {
+        std::fill(W.begin(), W.end(), 0);
+        std::fill(CS.begin(), CS.end(), 0);
+    }
     L.tiled = tiled;
     L.persistent = tiled && (nb == 8 || quad);
     L.quad = tiled && quad;
@@ -238,7 +289,7 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
     size_t off = 0;
     for (size_t b = 0; b < nbeams; ++b) {
         const BeamState& t = m_beams[b];
-        const size_t win = tiled ? (size_t)W[b] : 0;
+        const size_t win = (size_t)W[b];
         L.pitch[b] = round_up((round_up(std::max<size_t>(t.nout, 1), ubt) + t.tmax + spw - 1) / spw + win + 8, 32);
         // quad-strided rows are built straight from the input (K1d); the
         // channel-major packed copy exists only for the other forms
@@ -246,7 +297,10 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
         if (!L.quad) off += round_up((m_nchans + 1) * L.pitch[b], 64);
         if (L.quad) {
             // the tile windows read up to word (tiles - 1) * bt + tmax + P + 2
-            L.qpitch[b] = round_up(round_up(std::max<size_t>(t.nout, 1), ubt) + t.tmax + L.period + 4, 32);
+            // of a row (a pattern's series may start or end a few words past
+            // its trials' reads)
+            L.qpitch[b] =
+                round_up(round_up(std::max<size_t>(t.nout, 1), ubt) + t.tmax + L.period + (L.pattern ? 32 : 4), 32);
             L.q_off[b] = off;
             off += round_up((m_nchans + 1) * L.qpitch[b], 64);
         }
@@ -262,9 +316,9 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
         a.out_nbits = m_out_nbits;
         a.den = in_range * (float)m_nchans;
         a.factor = 3.f * 1024.f / 255.f / 16.f;
-        a.win_words = tiled ? W[b] : 0;
-        a.chan_per_stage = tiled ? CS[b] : 0;
-        a.nstages = tiled ? std::max(1, ((int)m_chan.size() + CS[b] - 1) / CS[b]) : 0;
+        a.win_words = W[b];
+        a.chan_per_stage = CS[b];
+        a.nstages = CS[b] ? std::max(1, ((int)m_chan.size() + CS[b] - 1) / CS[b]) : 0;
         a.variant = tiled ? v : 0;
         const size_t nbx = (t.sorted.size() + ubd - 1) / ubd;
         size_t nby = (t.nout + ubt - 1) / ubt;
@@ -276,7 +330,7 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
         L.nbx[b] = (int)nbx;
         L.units[b] = t.sorted.size() * covered;
         L.start[b + 1] = L.start[b] + (unsigned long long)(nbx * nby);
-        if (tiled) L.smem = std::max(L.smem, kern::tiled_batch_smem_bytes(nb, W[b], CS[b], v));
+        if (tiled && !L.pattern) L.smem = std::max(L.smem, kern::tiled_batch_smem_bytes(nb, W[b], CS[b], v));
     }
     L.ws_words = off;
     return L;
@@ -325,6 +379,7 @@ void TddBatch::upload(Layout& L)
         a.perm = t.perm.empty() ? nullptr : m_d_perm.get<int32_t>() + t.dm_off;
         a.out = t.spec.out;
         a.err = m_d_err.get<unsigned>();
+        if (L.pattern) m_tables[b]->fill(a, 0);
     }
     L.args = args;
     L.ws = ws;
@@ -371,7 +426,8 @@ void TddBatch::enqueue(cudaStream_t s, const Layout& L, bool timing)
     if (L.persistent) {
         kern::BatchLaunch bl{m_d_args.get<kern::DedisperseArgs>(), m_d_start.get<unsigned long long>(),
                              m_d_nbx.get<int>(), (int)m_beams.size(), L.start.back(), L.smem};
-        kern::launch_dedisperse_tiled_batch(bl, m_nbits, L.shape.variant, s);
+        if (L.pattern) kern::launch_dedisperse_pattern_batch(bl, m_nbits, m_lane_words, s);
+        else kern::launch_dedisperse_tiled_batch(bl, m_nbits, L.shape.variant, s);
         ++launches;
     } else {
         for (size_t b = 0; b < m_beams.size(); ++b) {

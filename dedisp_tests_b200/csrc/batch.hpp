@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "runtime.hpp"
+#include "tdd_engine.hpp"
 #include "tdd_kernels.hpp"
 
 namespace dedisp {
@@ -83,6 +84,7 @@ private:
     struct Layout;
     Layout make_layout(const BatchShape& shape, size_t tile_limit_samples) const;
     void upload(Layout& L);
+    void prepare_patterns();
     void enqueue(cudaStream_t s, const Layout& L, bool timing);
     void drop_graph();
     uint8_t* workspace_base();
@@ -101,6 +103,9 @@ private:
 
     rt::DeviceBuffer m_d_delay, m_d_chan, m_d_cdl, m_d_kmv, m_d_dms, m_d_perm, m_d_args, m_d_start, m_d_nbx;
     rt::DeviceBuffer m_d_err;  // set by a quad-strided kernel whose bounded wait expired
+    std::vector<std::unique_ptr<PatternTables>> m_tables;  // per beam, while the pattern kernel is used
+    bool m_pattern = false;    // the default shape runs the pattern kernel
+    int m_lane_words = 0;      // with this many words per lane
     rt::DeviceBuffer m_own_ws;
     void* m_ext_ws = nullptr;
     size_t m_ext_ws_bytes = 0;

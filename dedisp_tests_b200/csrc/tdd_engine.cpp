@@ -7,6 +7,7 @@
 
 #include "host_math.hpp"
 #include "tdd_kernels.hpp"
+#include "tdd_pattern.hpp"
 
 namespace dedisp {
 namespace detail {
@@ -17,6 +18,16 @@ constexpr int kMaxOutGroups = 8;                   // DM groups for D2H overlap
 size_t round_up(size_t a, size_t b) { return (a + b - 1) / b * b; }
 }  // namespace
 
+bool pattern_takes(const std::vector<float>& dms, const std::vector<float>& delays, int nbits)
+{
+    const size_t nact = delays.size();
+    if (nbits > 8 || nact == 0 || dms.empty()) return false;
+    if (nbits < 8 && nact * ((1u << nbits) - 1u) > 65535u) return false;
+    if (!(delays.front() >= 0.f) || !std::is_sorted(delays.begin(), delays.end())) return false;
+    if ((dms.size() + kern::kPatternDms - 1) / kern::kPatternDms > 65535) return false;
+    return hostmath::delay_rn(dms.back(), delays.back()) < (1u << 30);
+}
+
 // Everything derived from (DM list, killmask, DM range, nbits, kernel choice).
 struct TddEngine::Setup {
     unsigned long version = ~0ul;
@@ -25,9 +36,20 @@ struct TddEngine::Setup {
     TddKernel kernel = TddKernel::Auto;
     int variant = -1;
 
+    bool tiled_ok = false;       // a tiled form may run (0/1 killmask, not plain by choice)
+    bool pattern_ok = false;     // and the pattern kernel among them
+    long group_words = 0;        // widest group's row words beyond its periods (0: not known yet)
+    int table[3] = {0, 0, 0};    // pattern tables for 16, 8, 4 words per lane: 1 built, -1 rows are faster
+    bool rows_sized = false;     // row-by-row form: sizes below are set
+    bool rows_tiled = false, rows_quad = false;
+    int rows_period = 0;
+
+    // form of the current call
     bool tiled = false;
-    bool quad = false;           // 8-bit kernel on quad-strided rows
-    int period = 0;              // quad: P, words per lane set
+    bool quad = false;           // strided rows (quad kernels, pattern kernel)
+    bool pattern = false;        // shared channel-group sums (tdd_pattern.hpp)
+    int lane_words = 0;          // pattern: words per lane
+    int period = 0;              // strided rows: P, words per lane set
     int nact = 0;
     int win_words = 0;
     int chan_per_stage = 0;
@@ -39,6 +61,75 @@ struct TddEngine::Setup {
     std::vector<float> dms;      // ascending (tiled) or in list order (plain)
     std::vector<int32_t> perm;   // output row of each slot
 };
+
+void PatternTables::size(const float* d_dms, size_t ndm, const int32_t* d_chan, const float* d_delay, size_t nact,
+                         size_t zero_row, int nbits, int lane_words, cudaStream_t st)
+{
+    const size_t nblk = (ndm + kern::kPatternDms - 1) / kern::kPatternDms;
+    const size_t ngroups = (nact + kern::kPatternGroup - 1) / kern::kPatternGroup;
+    const size_t head = sizeof(kern::PatternTotals) + nblk * sizeof(uint4);
+    static_assert(sizeof(kern::PatternTotals) % sizeof(uint4) == 0, "block counts follow the totals");
+    m_sizes.reserve(head + nblk * ngroups * sizeof(int4));
+    m_nbits = nbits;
+    kern::PatternTableArgs a{};
+    a.dms = d_dms;
+    a.ndm = (int)ndm;
+    a.chan_list = d_chan;
+    a.chan_delay = d_delay;
+    a.nact = (int)nact;
+    a.zero_row = (int32_t)zero_row;
+    a.ngroups = (int)ngroups;
+    a.lane_words = lane_words;
+    a.period = 32 * lane_words;
+    a.series_words = kern::pattern_series_words(nbits);
+    a.series_width = kern::pattern_series_width(nbits);
+    a.ring_words = kern::pattern_ring_words(nbits);
+    a.run_words = kern::pattern_run_words(nbits);
+    a.build_warps = kern::pattern_build_warps(nbits, lane_words);
+    uint8_t* base = m_sizes.get<uint8_t>();
+    a.totals = reinterpret_cast<kern::PatternTotals*>(base);
+    a.block = reinterpret_cast<uint4*>(base + sizeof(kern::PatternTotals));
+    a.size = reinterpret_cast<int4*>(base + head);
+    kern::launch_pattern_sizes(a, st);
+    m_args = a;
+}
+
+PatternTables::Fit PatternTables::fit(cudaStream_t st)
+{
+    RT_CHECK(cudaMemcpyAsync(&m_total, m_args.totals, sizeof(m_total), cudaMemcpyDeviceToHost, st));
+    RT_CHECK(cudaStreamSynchronize(st));
+    if ((long)m_total.rows > kern::pattern_max_group_words(m_nbits)) return kTooWide;
+    // Wavefronts of the row-by-row kernel over the same tiles: one per trial,
+    // channel and 32 words, at a higher rate (256 channels, 512 trials 10
+    // samples apart, 2 bits: 0.240 ms here against 0.231 at nearly equal
+    // wavefronts; 5% below them the two are even).
+    const unsigned long long rows = (unsigned long long)m_args.ndm * m_args.nact * m_args.lane_words;
+    const size_t piece = sizeof(kern::PatternPiece) + 16 * sizeof(uint4) + (size_t)m_total.rec_words * 4;
+    return m_total.cost * 8 < rows * 7 && m_total.pieces * piece <= ((size_t)2 << 30) ? kUse : kRowsFaster;
+}
+
+void PatternTables::emit(cudaStream_t st)
+{
+    kern::PatternTableArgs& a = m_args;
+    const size_t n = m_total.pieces;
+    a.rec_stride = m_total.rec_words;
+    const size_t win = n * 16 * sizeof(uint4), rec = n * a.rec_stride * 4;  // 16-byte multiples
+    m_tables.reserve(win + rec + n * sizeof(kern::PatternPiece));
+    uint8_t* base = m_tables.get<uint8_t>();
+    a.win = reinterpret_cast<uint4*>(base);
+    a.rec = reinterpret_cast<uint32_t*>(base + win);
+    a.sched = reinterpret_cast<kern::PatternPiece*>(base + win + rec);
+    kern::launch_pattern_tables(a, m_total.pieces, st);
+}
+
+void PatternTables::fill(kern::DedisperseArgs& a, size_t block) const
+{
+    a.rec = m_args.rec;
+    a.rec_stride = m_args.rec_stride;
+    a.win = m_args.win;
+    a.block = m_args.block + block;
+    a.lane_words = m_args.lane_words;
+}
 
 TddEngine::TddEngine(GpuState& gpu) : m_gpu(gpu), m_setup(new Setup()) {}
 TddEngine::~TddEngine()
@@ -61,14 +152,18 @@ void TddEngine::prepare(const TddView& v, const TddCall& c)
 {
     Setup& s = *m_setup;
     // variants are numbered per input width; one outside the width's range
-    // (or -1) selects the width's default
+    // (or -1) selects the width's default, which is the pattern kernel where
+    // that is the faster one
     const int eff_variant = (variant >= 0 && variant < kern::tiled_variant_count(c.in_nbits))
                                 ? variant
                                 : kern::tiled_default_variant(c.in_nbits);
     if (s.version == v.version && s.first == c.first_dm && s.count == c.dm_count &&
-        s.nbits == c.in_nbits && s.kernel == kernel && s.variant == eff_variant)
+        s.nbits == c.in_nbits && s.kernel == kernel && s.variant == eff_variant) {
+        choose_form(v, c);
         return;
+    }
 
+    s.version = ~0ul;  // the tables below are rewritten
     Setup n;
     n.version = v.version;
     n.first = c.first_dm;
@@ -114,46 +209,17 @@ void TddEngine::prepare(const TddView& v, const TddCall& c)
         n.tmax = std::max(n.tmax, std::max(hostmath::delay_rn(dlo, dl), hostmath::delay_rn(dhi, dl)));
     }
 
-    n.tiled = (kernel != TddKernel::Plain) && !general;
-    if (n.tiled) {
-        const int bd = kern::tiled_block_dms(c.in_nbits, n.variant);
-        const int spw = 32 / c.in_nbits;
-        const int J = kern::tiled_lane_words(c.in_nbits, n.variant);
-        uint32_t span = 0;
-        for (size_t t = 0; t < c.dm_count; t += bd) {
-            const float f = n.dms[t], l = n.dms[std::min(t + bd, (size_t)c.dm_count) - 1];
-            for (int j = 0; j < n.nact; ++j) {
-                const float dl = v.delays[n.chan_list[j]];
-                const uint32_t a = hostmath::delay_rn(f, dl), b = hostmath::delay_rn(l, dl);
-                span = std::max(span, a > b ? a - b : b - a);
-            }
-        }
-        // quad-strided rows: a 1-sample delay is a 1-word offset, the window
-        // is the lane set (P words) plus the span plus the 16-byte rounding
-        n.quad = kern::tiled_variant_quad(c.in_nbits, n.variant);
-        n.period = 32 * J;
-        const size_t w = n.quad ? (size_t)span + 3 + (size_t)n.period
-                                : (span + 4 * (size_t)spw - 1) / spw + 32 * (size_t)J + 1;
-        n.win_words = (int)round_up(w, 4);
-        const int cs = w > ((size_t)1 << 26) ? 0 : kern::tiled_stage_channels(c.in_nbits, n.win_words, n.variant);
-        if (cs < 2) {
-            n.tiled = false;
-        } else {
-            n.chan_per_stage = cs;
-            n.nstages = std::max(1, (n.nact + cs - 1) / cs);
-        }
-    }
-    if (kernel == TddKernel::Tiled && !n.tiled)
-        DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "tiled kernel unavailable for this killmask/DM list");
-
+    n.tiled_ok = (kernel != TddKernel::Plain) && !general;
+    cudaStream_t st = m_gpu.stream();
     std::vector<int32_t> chan(n.chan_list);
-    if (n.tiled) chan.resize((size_t)n.nstages * n.chan_per_stage, (int32_t)v.nchans);
     if (chan.empty()) chan.push_back((int32_t)v.nchans);
     // delay of each list entry (the padding channel's is 0)
     std::vector<float> cdl(chan.size());
     for (size_t j = 0; j < chan.size(); ++j) cdl[j] = chan[j] < (int32_t)v.nchans ? v.delays[chan[j]] : 0.f;
-
-    cudaStream_t st = m_gpu.stream();
+    n.pattern_ok = n.tiled_ok && n.variant == kern::tiled_default_variant(c.in_nbits) && n.nact &&
+                   pattern_takes(n.dms, cdl, c.in_nbits);
+    m_dms.reserve(n.dms.size() * 4);
+    RT_CHECK(cudaMemcpyAsync(m_dms.get(), n.dms.data(), n.dms.size() * 4, cudaMemcpyHostToDevice, st));
     m_chan.reserve(chan.size() * 4);
     RT_CHECK(cudaMemcpyAsync(m_chan.get(), chan.data(), chan.size() * 4, cudaMemcpyHostToDevice, st));
     m_cdl.reserve(cdl.size() * 4);
@@ -162,8 +228,6 @@ void TddEngine::prepare(const TddView& v, const TddCall& c)
     if (km.empty()) km.push_back(0);
     m_km.reserve(km.size() * 4);
     RT_CHECK(cudaMemcpyAsync(m_km.get(), km.data(), km.size() * 4, cudaMemcpyHostToDevice, st));
-    m_dms.reserve(n.dms.size() * 4);
-    RT_CHECK(cudaMemcpyAsync(m_dms.get(), n.dms.data(), n.dms.size() * 4, cudaMemcpyHostToDevice, st));
     if (!n.identity) {
         m_perm.reserve(n.perm.size() * 4);
         RT_CHECK(cudaMemcpyAsync(m_perm.get(), n.perm.data(), n.perm.size() * 4,
@@ -172,6 +236,96 @@ void TddEngine::prepare(const TddView& v, const TddCall& c)
     // The host vectors must outlive the asynchronous copies.
     RT_CHECK(cudaStreamSynchronize(st));
     *m_setup = std::move(n);
+    choose_form(v, c);
+}
+
+// The form that this call takes (after prepare): the pattern kernel with the
+// period that suits the call's size where it is the faster one, else the
+// row-by-row kernel of the chosen variant, else the plain one.
+void TddEngine::choose_form(const TddView& v, const TddCall& c)
+{
+    Setup& s = *m_setup;
+    s.pattern = false;
+    // an explicitly tiled plan is refused where the row-by-row form is
+    if (kernel == TddKernel::Tiled) size_rows(v, c.in_nbits);
+    if (kernel == TddKernel::Tiled && !s.rows_tiled)
+        DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "tiled kernel unavailable for this killmask/DM list");
+    if (s.pattern_ok) {
+        const size_t nout = std::min(c.nsamps - v.max_delay, gulp_set && gulp_size ? gulp_size : kDefaultGulp);
+        const size_t bt = (size_t)kern::pattern_block_samples(c.in_nbits, 4);
+        const size_t tiles = (s.dms.size() + kern::kPatternDms - 1) / kern::kPatternDms * ((nout + bt - 1) / bt);
+        cudaStream_t st = m_gpu.stream();
+        int J = kern::pattern_lane_words(c.in_nbits, tiles, s.group_words), i = 0;
+        for (; J; J = kern::pattern_lane_words(c.in_nbits, tiles, s.group_words)) {
+            i = J == 16 ? 0 : J == 8 ? 1 : 2;
+            if (s.table[i]) break;
+            PatternTables& t = m_tables[i];
+            t.size(m_dms.get<float>(), s.dms.size(), m_chan.get<int32_t>(), m_cdl.get<float>(), (size_t)s.nact,
+                   v.nchans, c.in_nbits, J, st);
+            const PatternTables::Fit fit = t.fit(st);
+            s.group_words = t.group_words();
+            if (fit == PatternTables::kTooWide) continue;  // a shorter period, if one fits
+            s.table[i] = fit == PatternTables::kUse ? 1 : -1;
+            if (fit == PatternTables::kUse) t.emit(st);
+            break;
+        }
+        s.pattern = J && s.table[i] == 1;
+        s.lane_words = J;
+    }
+    if (!s.pattern) size_rows(v, c.in_nbits);
+    s.tiled = s.pattern || s.rows_tiled;
+    s.quad = s.pattern || s.rows_quad;
+    s.period = s.pattern ? 32 * s.lane_words : s.rows_period;
+}
+
+// Window and stage sizes of the row-by-row tiled form, and its padded channel
+// list.
+void TddEngine::size_rows(const TddView& v, int nbits)
+{
+    Setup& s = *m_setup;
+    if (s.rows_sized) return;
+    s.rows_tiled = s.tiled_ok;
+    if (s.rows_tiled) {
+        const size_t ndm = s.dms.size();
+        const int bd = kern::tiled_block_dms(nbits, s.variant);
+        const int spw = 32 / nbits;
+        const int J = kern::tiled_lane_words(nbits, s.variant);
+        uint32_t span = 0;
+        for (size_t t = 0; t < ndm; t += bd) {
+            const float f = s.dms[t], l = s.dms[std::min(t + bd, ndm) - 1];
+            for (int j = 0; j < s.nact; ++j) {
+                const float dl = v.delays[s.chan_list[j]];
+                const uint32_t a = hostmath::delay_rn(f, dl), b = hostmath::delay_rn(l, dl);
+                span = std::max(span, a > b ? a - b : b - a);
+            }
+        }
+        // quad-strided rows: a 1-sample delay is a 1-word offset, the window
+        // is the lane set (P words) plus the span plus the 16-byte rounding
+        s.rows_quad = kern::tiled_variant_quad(nbits, s.variant);
+        s.rows_period = 32 * J;
+        const size_t w = s.rows_quad ? (size_t)span + 3 + (size_t)s.rows_period
+                                     : (span + 4 * (size_t)spw - 1) / spw + 32 * (size_t)J + 1;
+        s.win_words = (int)round_up(w, 4);
+        const int cs = w > ((size_t)1 << 26) ? 0 : kern::tiled_stage_channels(nbits, s.win_words, s.variant);
+        if (cs < 2) {
+            s.rows_tiled = s.rows_quad = false;
+        } else {
+            s.chan_per_stage = cs;
+            s.nstages = std::max(1, (s.nact + cs - 1) / cs);
+            std::vector<int32_t> chan(s.chan_list);
+            chan.resize((size_t)s.nstages * s.chan_per_stage, (int32_t)v.nchans);
+            std::vector<float> cdl(chan.size());
+            for (size_t j = 0; j < chan.size(); ++j) cdl[j] = chan[j] < (int32_t)v.nchans ? v.delays[chan[j]] : 0.f;
+            cudaStream_t st = m_gpu.stream();
+            RT_CHECK(cudaStreamSynchronize(st));  // earlier calls read the shorter list
+            m_chan.reserve(chan.size() * 4);
+            m_cdl.reserve(cdl.size() * 4);
+            RT_CHECK(cudaMemcpyAsync(m_chan.get(), chan.data(), chan.size() * 4, cudaMemcpyHostToDevice, st));
+            RT_CHECK(cudaMemcpyAsync(m_cdl.get(), cdl.data(), cdl.size() * 4, cudaMemcpyHostToDevice, st));
+            RT_CHECK(cudaStreamSynchronize(st));
+        }
+    }
+    s.rows_sized = true;
 }
 
 void TddEngine::execute(const TddView& v, const TddCall& c)
@@ -196,8 +350,10 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     if (dev_out && c.out_stride % ob != 0)
         DD_THROW_MSG(DEDISP_INVALID_STRIDE, "device output stride must be a multiple of the sample size");
 
-    const size_t bt = s.tiled ? (size_t)kern::tiled_block_samples(nbits, s.variant) : 16;
-    const size_t win = s.tiled ? (size_t)s.win_words : 0;
+    const size_t bt = s.pattern ? (size_t)kern::pattern_block_samples(nbits, s.lane_words)
+                      : s.tiled ? (size_t)kern::tiled_block_samples(nbits, s.variant)
+                                : 16;
+    const size_t win = s.tiled && !s.pattern ? (size_t)s.win_words : 0;
 
     // Gulp size: the user cap, the grid limit, then device memory. With more
     // than one gulp the input rows and the output rows of a gulp have two
@@ -211,9 +367,11 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
         return round_up((round_up(g, bt) + s.tmax + spw - 1) / spw + win + 8, 32);
     };
     // quad-strided rows: the tile windows read up to word
-    // (tiles - 1) * bt + tmax + P + 2 of a row
+    // (tiles - 1) * bt + tmax + P + 2 of a row (a pattern's series may start
+    // or end a few words past its trials' reads)
     const bool quad = s.tiled && s.quad;
-    auto qpitch_for = [&](size_t g) { return round_up(round_up(g, bt) + s.tmax + s.period + 4, 32); };
+    const size_t slack = s.pattern ? 32 : 4;
+    auto qpitch_for = [&](size_t g) { return round_up(round_up(g, bt) + s.tmax + s.period + slack, 32); };
     auto nbuf_for = [&](size_t g) -> size_t { return nsamp_out > g ? 2 : 1; };
     auto in_bytes_for = [&](size_t g) { return round_up(g + s.tmax, 128) * row_bytes; };
     // quad-strided rows are built straight from the input rows (K1d); the
@@ -258,7 +416,7 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     // contiguous, so that its device-to-host copy starts group by group
     // (every other gulp's copy already overlaps the next gulp's kernels, and
     // each extra launch ends with a partly filled wave).
-    const size_t bd = s.tiled ? (size_t)kern::tiled_block_dms(nbits, s.variant) : 32;
+    const size_t bd = s.tiled && !s.pattern ? (size_t)kern::tiled_block_dms(nbits, s.variant) : 32;
     const size_t ntile = (ndm + bd - 1) / bd;
     const size_t ngroups_last = (!dev_out && s.identity) ? std::min<size_t>(kMaxOutGroups, ntile) : 1;
 
@@ -367,7 +525,10 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
                 da.perm = m_perm.get<int32_t>() + s0;
                 da.out = out_base;
             }
-            if (s.tiled) kern::launch_dedisperse_tiled(da, ex);
+            if (s.pattern) {
+                m_tables[s.lane_words == 16 ? 0 : s.lane_words == 8 ? 1 : 2].fill(da, s0 / bd);  // s0 is a multiple of bd
+                kern::launch_dedisperse_pattern(da, ex);
+            } else if (s.tiled) kern::launch_dedisperse_tiled(da, ex);
             else kern::launch_dedisperse_plain(da, ex);
             ++stats.launches;
             if (!dev_out) event(ev + groups.size() - 1).record(ex);

@@ -17,6 +17,8 @@
 #include <vector>
 
 #include "gpu_state.hpp"
+#include "tdd_kernels.hpp"
+#include "tdd_pattern.hpp"
 #include "tdd/TDDPlan.hpp"
 
 namespace dedisp {
@@ -54,6 +56,36 @@ struct TddStats {
     bool tiled = false;
 };
 
+// Whether the pattern kernel takes these (ascending) DMs and active channels'
+// delays: it needs ascending delays (no channel of a group is delayed less than
+// its first) and sums that its narrow lanes hold.
+bool pattern_takes(const std::vector<float>& dms, const std::vector<float>& delays, int nbits);
+
+// The pattern kernel's device tables for one DM list and channel list: size()
+// enqueues the size pass for a period, fit() reads its totals and emit()
+// enqueues the tables.
+class PatternTables {
+public:
+    void size(const float* d_dms, size_t ndm, const int32_t* d_chan, const float* d_delay, size_t nact,
+              size_t zero_row, int nbits, int lane_words, cudaStream_t st);
+    enum Fit { kUse, kRowsFaster, kTooWide };
+    // kTooWide: some group's rows do not fit the ring at this period (try a
+    // shorter one); kRowsFaster: the row-by-row kernel needs fewer
+    // shared-memory wavefronts, or the tables exceed 2 GiB. Waits for `st`.
+    Fit fit(cudaStream_t st);
+    // Row words of the widest group beyond its periods (after fit).
+    long group_words() const { return (long)m_total.rows - (long)kern::kPatternGroup * 32 * m_args.lane_words; }
+    void emit(cudaStream_t st);
+    // Table arguments for the DM blocks from `block` on.
+    void fill(kern::DedisperseArgs& a, size_t block) const;
+
+private:
+    rt::DeviceBuffer m_sizes, m_tables;
+    kern::PatternTableArgs m_args{};
+    kern::PatternTotals m_total{};
+    int m_nbits = 0;
+};
+
 class TddEngine {
 public:
     // Gulp (output samples per pass) unless set: device-resident calls take
@@ -77,10 +109,13 @@ public:
 private:
     struct Setup;
     void prepare(const TddView& v, const TddCall& c);
+    void choose_form(const TddView& v, const TddCall& c);
+    void size_rows(const TddView& v, int nbits);
 
     GpuState& m_gpu;
     std::unique_ptr<Setup> m_setup;
     rt::DeviceBuffer m_chan, m_cdl, m_km, m_dms, m_perm, m_tr, m_q, m_out[2], m_stage[2];
+    PatternTables m_tables[3];  // 16, 8, 4 words per lane
     rt::DeviceBuffer m_err;  // set by a quad-strided kernel whose bounded wait expired
     std::vector<std::unique_ptr<rt::Event>> m_events;
     rt::Event& event(size_t i);

@@ -56,6 +56,12 @@ struct DedisperseArgs {
     int variant;                // tiled: tile-shape variant (8-bit input)
     unsigned* err;              // quad-strided: device word set to 1 when a bounded
                                 // wait on the staged copies expired (required)
+    // shared channel-group sums (tdd_pattern.hpp): tables per DM block
+    const uint32_t* rec;
+    size_t rec_stride;          // words
+    const uint4* win;
+    const uint4* block;
+    int lane_words;
 };
 
 // Tile geometry of the tiled kernel for a given input width and tile-shape

@@ -31,7 +31,9 @@ dedisp_error dedisp_b200_set_tdd_kernel(dedisp_plan plan, int kernel);
  * widened to bytes); 16/32-bit 0 only. Quad-strided rows are built per gulp
  * (four bytes per sample and channel in device memory). A variant outside
  * the executed width's range selects that width's default (quad-strided
- * 20 words x 12 DMs for widths up to 8 bits). Every variant computes the same
+ * 20 words x 12 DMs for widths up to 8 bits). The default variant, set or not,
+ * runs the kernel on shared channel-group sums (csrc/tdd_pattern.hpp) where that
+ * is the faster one for the DM list. Every variant computes the same
  * bit-exact sums; they differ in speed. */
 dedisp_error dedisp_b200_set_tdd_variant(dedisp_plan plan, int variant);
 int dedisp_b200_tdd_variant_count(dedisp_size in_nbits);
@@ -181,7 +183,9 @@ dedisp_error dedisp_b200_batch_set_workspace(dedisp_b200_batch batch, void* d_wo
                                              dedisp_size bytes);
 /* Tile shape: variant < dedisp_b200_batch_variant_count(in_nbits), channels
  * per stage even and <= 32 (0: the largest that fits shared memory; the
- * quad-strided variants size their stages per block and ignore it). */
+ * quad-strided variants size their stages per block and ignore it). The default
+ * variant with 0 runs the kernel on shared channel-group sums where that is the
+ * faster one for every beam. */
 int dedisp_b200_batch_variant_count(dedisp_size in_nbits);
 dedisp_error dedisp_b200_batch_set_shape(dedisp_b200_batch batch, int variant, int chan_per_stage);
 /* Times every candidate shape on the leading 8192 output samples of each
