@@ -21,8 +21,9 @@ size_t round_up(size_t a, size_t b) { return (a + b - 1) / b * b; }
 bool pattern_takes(const std::vector<float>& dms, const std::vector<float>& delays, int nbits)
 {
     const size_t nact = delays.size();
-    if (nbits > 8 || nact == 0 || dms.empty()) return false;
-    if (nbits < 8 && nact * ((1u << nbits) - 1u) > 65535u) return false;
+    if (nbits > 16 || nact == 0 || dms.empty()) return false;
+    if (nbits < 8 && nact * ((1u << nbits) - 1u) > 65535u) return false;  // 16-bit lanes
+    if (nbits == 16 && nact > 65536u) return false;                       // 32-bit sums
     if (!(delays.front() >= 0.f) || !std::is_sorted(delays.begin(), delays.end())) return false;
     if ((dms.size() + kern::kPatternDms - 1) / kern::kPatternDms > 65535) return false;
     return hostmath::delay_rn(dms.back(), delays.back()) < (1u << 30);

@@ -658,6 +658,50 @@ __global__ void __launch_bounds__(QD_THREADS) quad_direct_kernel(QuadDirectArgs 
     }
 }
 
+// The same for 16-bit input: word n of a row holds samples n and n + P. A block
+// takes 16 input words (32 channels) of every row and 128 output words; each
+// thread turns one word of the two windows into output word n of two channels.
+__global__ void __launch_bounds__(QD_THREADS) pair_direct_kernel(QuadDirectArgs a, int aligned)
+{
+    constexpr int LOADS = 2 * QD_N * QD_WORDS / QD_THREADS;
+    __shared__ uint32_t tile[2][QD_N][QD_WORDS + 1];
+    const size_t n0 = (size_t)blockIdx.x * QD_N;
+    const size_t w0 = (size_t)blockIdx.y * QD_WORDS;
+    const size_t row_words = a.nchans / 2;
+    const size_t P = (size_t)a.period_words;
+
+    uint32_t v[LOADS];
+#pragma unroll
+    for (int it = 0; it < LOADS; ++it) {
+        const int idx = threadIdx.x + it * QD_THREADS;
+        const int k = idx % QD_WORDS, r = (idx / QD_WORDS) % QD_N, i = idx / (QD_WORDS * QD_N);
+        const size_t row = n0 + r + (size_t)i * P, wi = w0 + k;
+        v[it] = 0u;
+        if (row < a.rows_valid && wi < row_words) {
+            const uint8_t* p = a.in + row * a.in_pitch + wi * 4;
+            v[it] = aligned ? __ldg(reinterpret_cast<const uint32_t*>(p))
+                            : (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) |
+                                  ((uint32_t)p[3] << 24);
+        }
+    }
+#pragma unroll
+    for (int it = 0; it < LOADS; ++it) {
+        const int idx = threadIdx.x + it * QD_THREADS;
+        tile[idx / (QD_WORDS * QD_N)][(idx / QD_WORDS) % QD_N][idx % QD_WORDS] = v[it];
+    }
+    __syncthreads();
+
+    for (int item = threadIdx.x; item < QD_WORDS * QD_N; item += QD_THREADS) {
+        const int r = item % QD_N, k = item / QD_N;
+        const size_t n = n0 + r, c = 2 * (w0 + k);
+        if (n >= a.q_pitch_words || c >= a.nchans) continue;
+        const uint32_t e0 = tile[0][r][k], e1 = tile[1][r][k];
+        uint32_t* dst = a.q + c * a.q_pitch_words + n;
+        dst[0] = __byte_perm(e0, e1, 0x5410);
+        dst[a.q_pitch_words] = __byte_perm(e0, e1, 0x7632);
+    }
+}
+
 // Tile shapes of the quad-strided kernel: J words per lane (P = 32J), NW warps
 // = NW DMs per block (one DM per warp).
 struct Q8Shape { int J, NW; };
@@ -1168,7 +1212,8 @@ void launch_quad_direct(const QuadDirectArgs& a, cudaStream_t s)
     case 2: quad_direct_kernel<2><<<grid, QD_THREADS, 0, s>>>(a, aligned); break;
     case 4: quad_direct_kernel<4><<<grid, QD_THREADS, 0, s>>>(a, aligned); break;
     case 8: quad_direct_kernel<8><<<grid, QD_THREADS, 0, s>>>(a, aligned); break;
-    default: DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "quad-strided rows hold samples of at most 8 bits");
+    case 16: pair_direct_kernel<<<grid, QD_THREADS, 0, s>>>(a, aligned); break;
+    default: DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "strided rows hold samples of at most 16 bits");
     }
     RT_CHECK(cudaGetLastError());
 }

@@ -84,16 +84,16 @@ size_t tiled_batch_smem_bytes(int nbits, int win_words, int chan_per_stage, int 
 // Channels per pipeline stage for a window of win_words (0: does not fit).
 int tiled_stage_channels(int nbits, int win_words, int variant);
 
-// K1d: quad-strided rows straight from time-major packed 1/2/4/8-bit input:
+// K1d: quad-strided rows straight from time-major packed 1/2/4/8/16-bit input:
 // rows 0..nchans-1 of q, word n of channel c holding samples n + i*P
-// (i = 0..3) of the channel as bytes, zero at or past rows_valid. The
-// all-zero padding row is the caller's.
+// (i = 0..3) of the channel as bytes (16-bit input: samples n and n + P as
+// halves), zero at or past rows_valid. The all-zero padding row is the caller's.
 struct QuadDirectArgs {
     const uint8_t* in;    // input row t at in + t * in_pitch
     size_t in_pitch;      // bytes
     size_t rows_valid;    // rows present in `in`
     size_t nchans;
-    int nbits;            // 1, 2, 4 or 8
+    int nbits;            // 1, 2, 4, 8 or 16
     uint32_t* q;          // quad-strided rows, q_pitch_words apart
     size_t q_pitch_words; // words per row (a multiple of 4), all written
     int period_words;     // P, a multiple of 4

@@ -16,7 +16,7 @@ FINE = (64e-6, 1300.0, -0.078125)   # dt, f0, df: wide spans per trial
 COARSE = (250e-6, 1500.0, -0.5)
 
 
-@pytest.mark.parametrize("nbits", [1, 2, 4, 8])
+@pytest.mark.parametrize("nbits", [1, 2, 4, 8, 16])
 @pytest.mark.parametrize("setup,nchans,ndm,dm_lo,dm_hi,nout,gulp", [
     (COARSE, 64, 1, 40.0, 40.0, 700, 0),          # one trial, a few short tiles
     (COARSE, 32, 31, 0.0, 30.0, 2049, 0),         # trials fill most of one block
