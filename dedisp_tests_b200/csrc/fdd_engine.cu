@@ -160,20 +160,23 @@ void FddEngine::execute(const FddOptions& opt, const FddView& v, const FddCall& 
     bool tc_direct = false, tc_hybrid = false;
     int tc_form = -1;
     const int seg_group = (int)std::min<size_t>(nseg, (size_t)kern::kTcMaxSeg);
-    if (use_tc || nseg == 1) {
+    {
         // Largest delay index over all DMs and active channels (same float
-        // operations as the kernels): the tensor-core MAC and the one-segment
-        // FP32 MAC build a per-bin phasor table over 0..dmax when it fits
-        // shared memory.
+        // operations as the kernels): both MACs build a per-bin phasor table
+        // over 0..dmax when it fits shared memory.
         const int rnd = opt.round_delays ? 1 : 0;
         if (m.dmax_version != v.version || m.dmax_round != rnd) {
+            // (the largest DM: products are monotonic in dm >= 0)
             long dmax = 0;
             bool ok = true;
+            float top = 0.f;
             for (size_t i = 0; i < ndm && ok; ++i) {
-                const float d = v.dms[i];
-                if (!(d >= 0.f)) { ok = false; break; }
+                ok = v.dms[i] >= 0.f;
+                top = std::max(top, v.dms[i]);
+            }
+            if (ok) {
                 for (float dl : m.delays_active) {
-                    const long x = rnd ? (long)hostmath::delay_rn(d, dl) : (long)hostmath::delay_trunc(d, dl);
+                    const long x = rnd ? (long)hostmath::delay_rn(top, dl) : (long)hostmath::delay_trunc(top, dl);
                     dmax = std::max(dmax, x);
                 }
             }
@@ -321,11 +324,10 @@ void FddEngine::execute(const FddOptions& opt, const FddView& v, const FddCall& 
         a.nfft = (unsigned)g.nfft;
         a.round_delays = opt.round_delays ? 1 : 0;
         a.tw = tw;
-        // one segment: the per-bin phasor table (each phasor feeds one
-        // product); several: the tiled kernel, which reuses each phasor
-        // across the segments
-        if (nseg == 1 && kern::fdd_mac_series_fits(m.dmax, (unsigned)g.nfft, m.nact))
-            kern::launch_fdd_mac_series(a, m.dmax, st);
+        // the per-bin phasor table where it fits (DMs without negative delays,
+        // max delays up to about 20000), else phasors from the twiddle tables
+        if (kern::fdd_mac_table_fits(m.dmax, (unsigned)g.nfft, (int)ndm, m.nact, (int)nseg))
+            kern::launch_fdd_mac_table(a, m.dmax, st);
         else
             kern::launch_fdd_mac_plain(a, st);
         stats.launches = 1;

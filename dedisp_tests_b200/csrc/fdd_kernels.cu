@@ -1184,86 +1184,139 @@ __global__ void __launch_bounds__(MAC_THREADS) mac_plain_kernel(MacArgs a, int b
     }
 }
 
-// FP32 MAC for one segment (the whole-series forms): each phasor feeds a
-// single product, so generating it is the work. Per bin the CTA builds the
-// phasors of every delay 0..dmax in shared memory (index k d mod N stepped
-// exactly by (k S) mod N, the same phasor() product as the tiled kernel), loads
-// the bin's spectra, and each thread accumulates SERIES_DPT DMs over all
-// channels, in the tiled kernel's channel order and FMA sequence (so the sums
-// are the same). Delays: dm * delay rounded by adding 2^23 (toward zero, or to
-// nearest even), exact for 0 <= dm * delay < 2^22 (dmax bounds it).
-constexpr int SERIES_THREADS = 256;
-constexpr int SERIES_DPT = 8;  // DMs per thread and pass
+// FP32 MAC with a phasor table per bin: the form that runs whenever every delay
+// index 0..dmax fits shared memory. Per bin the CTA builds the phasors of all
+// delays (index k d mod N stepped exactly by (k nt) mod N, the same phasor()
+// product as the tiled kernel), then each thread accumulates TM DMs x TS
+// segments over all channels, in the tiled kernel's channel order and FMA
+// sequence, so the sums are the same bit for bit. A phasor costs a delay (dm *
+// delay rounded by adding 2^23, toward zero or to nearest even: exact for 0 <=
+// dm * delay < 2^22, which dmax bounds) and one shared load that neighbouring
+// DMs take from neighbouring entries, and feeds 2 TS packed FMAs; the channel's
+// spectra are 8-byte broadcasts. (A broadcast still returns 32 lanes' worth of
+// data at 128 bytes a cycle: (x, y, y, x) as 16 bytes with two DMs a thread held
+// the FMA pipe at 44%.)
+//
+// Bound by FMA and other issue (58% of the FMA pipe at 9 segments: 4 TM TS FMAs
+// against 5 TM + 2 TS other instructions per channel), at one segment by shared
+// loads and issue alike. Segments are taken in equal tiles of at most 10: the
+// tiled kernel's 40-wide tile multiplied 31 columns of padding at 9 segments,
+// and computed each phasor from the twiddle tables. Packed fma.rn.f32x2 was
+// slower (20.1 ms against 14.4 at 9 segments): two moves per FMA to build its
+// operand pairs.
+// Measured on B200, 1024 channels, ms, tiled (one segment: 8 DMs a thread of 256)
+// -> here: 512 DMs x 16385 bins x 9 segments 74.6 -> 14.4; 2048 DMs x 39 segments
+// 336 -> 255; 512 DMs x 73728 bins x 1 segment 56.7 -> 17.9.
+constexpr int TAB_THREADS = 256;
+constexpr int TAB_CK = 128;      // channels staged at a time
+constexpr int TAB_MAX_TS = 10;
 
-__global__ void __launch_bounds__(SERIES_THREADS) mac_series_kernel(MacArgs a, int dmax, int bins_per_block)
+__device__ __forceinline__ float2 lds_float2(uint32_t addr)
 {
-    extern __shared__ __align__(16) float2 s_ser[];
-    const unsigned tab_n = ((unsigned)dmax + 2u) & ~1u;  // even counts keep the float2 arrays aligned
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+
+template <int TS, int TM>
+__global__ void __launch_bounds__(TAB_THREADS) mac_table_kernel(MacArgs a, int dmax, int bins_per_block, int ts, int groups)
+{
+    extern __shared__ __align__(16) float2 s_tab[];
+    const unsigned tab_n = ((unsigned)dmax + 2u) & ~1u;  // even counts keep the arrays aligned
     const unsigned nhi = a.nfft / 256;
-    float2* table = s_ser;
+    float2* table = s_tab;
     float2* lo = table + tab_n;
     float2* hi = lo + 256;
-    float2* xs = hi + ((nhi + 1u) & ~1u);
-    float* dl = reinterpret_cast<float*>(xs + ((a.nact + 1) & ~1));
-    const int tid = threadIdx.x;
-    for (unsigned i = tid; i < 256; i += SERIES_THREADS) lo[i] = a.tw.lo[i];
-    for (unsigned i = tid; i < nhi; i += SERIES_THREADS) hi[i] = a.tw.hi[i];
-    for (int i = tid; i < a.nact; i += SERIES_THREADS) dl[i] = a.delay_act[i];
+    const int width = TS * groups;                              // columns staged, ts used of each TS
+    float2* xs = hi + ((nhi + 1u) & ~1u);                       // [TAB_CK][width]
+    float* dl = reinterpret_cast<float*>(xs + TAB_CK * width);  // [TAB_CK]
+    const int tid = threadIdx.x, nt = blockDim.x;
+    // thread = (segment group, DM thread); whole warps share a group
+    const int ndt = nt / groups, group = tid / ndt, dt = tid - group * ndt;
+    for (unsigned i = tid; i < 256; i += nt) lo[i] = a.tw.lo[i];
+    for (unsigned i = tid; i < nhi; i += nt) hi[i] = a.tw.hi[i];
     const bool rn = a.round_delays != 0;
-    const uint32_t dcap = (uint32_t)dmax;
+    // table entry d at table_d0 + 8 * (bits of 2^23 + d)
+    const uint32_t table_d0 = (uint32_t)__cvta_generic_to_shared(table) - 8u * 0x4B000000u;
 
     const size_t kb0 = (size_t)blockIdx.x * bins_per_block;
     const size_t kb1 = min(a.nbins, kb0 + bins_per_block);
     for (size_t k = kb0; k < kb1; ++k) {
-        __syncthreads();  // the previous bin's table and spectra are no longer read
+        __syncthreads();  // the previous bin's table is no longer read
         {
-            constexpr uint32_t S = SERIES_THREADS;
             uint32_t idx = (uint32_t)(((uint64_t)k * (uint64_t)tid) % a.nfft);
-            const uint32_t step = (uint32_t)(((uint64_t)k * S) % a.nfft);
-            for (int d = tid; d <= dmax; d += S) {
+            const uint32_t step = (uint32_t)(((uint64_t)k * (uint64_t)nt) % a.nfft);
+            for (int d = tid; d <= dmax; d += nt) {
                 table[d] = phasor(lo, hi, idx);
                 idx = (idx + step >= a.nfft) ? idx + step - a.nfft : idx + step;
             }
         }
-        for (int i = tid; i < a.nact; i += SERIES_THREADS) xs[i] = a.Xt[k * (size_t)a.nact + i];
-        __syncthreads();
-        for (int m0 = 0; m0 < a.ndm; m0 += SERIES_THREADS * SERIES_DPT) {
-            float dmv[SERIES_DPT];
-            float2 acc[SERIES_DPT];
+        for (int s0 = 0; s0 < a.nseg; s0 += ts * groups) {
+            const int sg = s0 + group * ts;             // this thread's first segment
+            const int ns = min(ts, a.nseg - sg);        // (none: <= 0)
+            for (int m0 = 0; m0 < a.ndm; m0 += ndt * TM) {
+                float dmv[TM];
+                float2 acc[TM][TS];
 #pragma unroll
-            for (int q = 0; q < SERIES_DPT; ++q) {
-                dmv[q] = a.dms[min(m0 + tid + q * SERIES_THREADS, a.ndm - 1)];
-                acc[q] = make_float2(0.f, 0.f);
-            }
-#pragma unroll 2
-            for (int c = 0; c < a.nact; ++c) {
-                const float delay = dl[c];
-                const float2 bv = xs[c];
+                for (int q = 0; q < TM; ++q) {
+                    dmv[q] = a.dms[min(m0 + dt + q * ndt, a.ndm - 1)];
 #pragma unroll
-                for (int q = 0; q < SERIES_DPT; ++q) {
-                    const float x = __fmul_rn(dmv[q], delay);
-                    const float y = rn ? __fadd_rn(x, 8388608.0f) : __fadd_rz(x, 8388608.0f);
-                    const float2 av = table[min(__float_as_uint(y) - 0x4B000000u, dcap)];
-                    acc[q].x = fmaf(av.x, bv.x, acc[q].x);
-                    acc[q].x = fmaf(-av.y, bv.y, acc[q].x);
-                    acc[q].y = fmaf(av.x, bv.y, acc[q].y);
-                    acc[q].y = fmaf(av.y, bv.x, acc[q].y);
+                    for (int s = 0; s < TS; ++s) acc[q][s] = make_float2(0.f, 0.f);
                 }
-            }
+                for (int c0 = 0; c0 < a.nact; c0 += TAB_CK) {
+                    const int nc = min(TAB_CK, a.nact - c0);
+                    __syncthreads();  // the staged channels are no longer read
+                    for (int i = tid; i < TAB_CK * width; i += nt) {
+                        const int col = i / TAB_CK, c = i - col * TAB_CK;
+                        const int g = col / TS, s = col - g * TS, seg = s0 + g * ts + s;
+                        float2 v = make_float2(0.f, 0.f);
+                        if (s < ts && seg < a.nseg && c < nc) v = a.Xt[(k * a.nseg + seg) * (size_t)a.nact + c0 + c];
+                        xs[c * width + col] = v;
+                    }
+                    for (int i = tid; i < nc; i += nt) dl[i] = a.delay_act[c0 + i];
+                    __syncthreads();
+                    const float2* xc = xs + group * TS;
+#pragma unroll 2
+                    for (int c = 0; c < nc; ++c, xc += width) {
+                        const float delay = dl[c];
+                        float2 av[TM];
 #pragma unroll
-            for (int q = 0; q < SERIES_DPT; ++q) {
-                const int m = m0 + tid + q * SERIES_THREADS;
-                if (m < a.ndm) a.Yt[k * (size_t)a.ndm + m] = acc[q];
+                        for (int q = 0; q < TM; ++q) {
+                            const float x = __fmul_rn(dmv[q], delay);
+                            const float y = rn ? __fadd_rn(x, 8388608.0f) : __fadd_rz(x, 8388608.0f);
+                            // 2^23 + d: d in the low mantissa bits
+                            av[q] = lds_float2(table_d0 + 8u * __float_as_uint(y));
+                        }
+#pragma unroll
+                        for (int s = 0; s < TS; ++s) {
+                            const float2 b = xc[s];
+#pragma unroll
+                            for (int q = 0; q < TM; ++q) {
+                                acc[q][s].x = fmaf(av[q].x, b.x, acc[q][s].x);
+                                acc[q][s].x = fmaf(-av[q].y, b.y, acc[q][s].x);
+                                acc[q][s].y = fmaf(av[q].x, b.y, acc[q][s].y);
+                                acc[q][s].y = fmaf(av[q].y, b.x, acc[q][s].y);
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < TM; ++q) {
+                    const int m = m0 + dt + q * ndt;
+                    if (m >= a.ndm) continue;
+#pragma unroll
+                    for (int s = 0; s < TS; ++s)
+                        if (s < ns) a.Yt[(k * a.nseg + sg + s) * (size_t)a.ndm + m] = acc[q][s];
+                }
             }
         }
     }
 }
 
-size_t series_smem_bytes(int dmax, unsigned nfft, int nact)
+size_t table_smem_bytes(int dmax, unsigned nfft, int columns)
 {
-    return ((size_t)(((unsigned)dmax + 2u) & ~1u) + 256 + ((nfft / 256 + 1) & ~1u) + (size_t)((nact + 1) & ~1)) *
-               sizeof(float2) +
-           (size_t)nact * sizeof(float);
+    return ((size_t)(((unsigned)dmax + 2u) & ~1u) + 256 + ((nfft / 256 + 1) & ~1u)) * sizeof(float2) +
+           (size_t)TAB_CK * (columns * sizeof(float2) + sizeof(float));
 }
 
 // CTAs of one wave of a persistent kernel: resident CTAs per SM x SMs,
@@ -1560,21 +1613,82 @@ void launch_fdd_spectrum_out(const float2* Yt, size_t ndm, size_t nspec, float* 
     RT_CHECK(cudaGetLastError());
 }
 
-bool fdd_mac_series_fits(int dmax, unsigned nfft, int nact)
+namespace {
+// Threads over DMs first; where those are too few to build the table (40
+// entries a thread) groups of threads take segments of their own.
+struct TableShape {
+    int tm, ndt, ts, groups;
+    TableShape(int ndm, int nseg, int dmax)
+    {
+        tm = nseg == 1 && ndm > 4 * TAB_THREADS ? 8 : ndm >= 128 ? 4 : ndm >= 64 ? 2 : 1;
+        ndt = std::min(TAB_THREADS, ((ndm + tm - 1) / tm + 31) / 32 * 32);
+        const int most = std::max(1, std::min(TAB_THREADS, dmax / 40) / ndt);
+        const int passes = (nseg + TAB_MAX_TS * most - 1) / (TAB_MAX_TS * most);
+        ts = (nseg + passes * most - 1) / (passes * most);
+        groups = std::min(most, (nseg + ts - 1) / ts);
+    }
+};
+}  // namespace
+
+bool fdd_mac_table_fits(int dmax, unsigned nfft, int ndm, int nact, int nseg)
 {
-    return dmax >= 0 && dmax < (1 << 22) && series_smem_bytes(dmax, nfft, nact) <= 200 * 1024;
+    if (dmax < 0 || dmax >= (1 << 22) || nfft % 256 != 0 || nseg < 1 || ndm < 1) return false;
+    // more table entries than phasors used: with enough segments for its tile
+    // the tiled kernel is the faster one (64 DMs x 256 channels x 49 segments,
+    // 18347 delays: 5.3 ms against 7.5)
+    if (nseg > TAB_MAX_TS && (long)dmax > (long)ndm * nact) return false;
+    const TableShape t(ndm, nseg, dmax);
+    return table_smem_bytes(dmax, nfft, t.ts * t.groups) <= 200 * 1024;
 }
 
-void launch_fdd_mac_series(const MacArgs& a, int dmax, cudaStream_t s)
+namespace {
+template <int TS, int TM>
+void launch_mac_table(const MacArgs& a, int dmax, int ts, int ndt, int groups, cudaStream_t s)
 {
-    if (a.nseg != 1 || !fdd_mac_series_fits(dmax, a.nfft, a.nact) || a.nfft % 256 != 0)
-        DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "one-segment MAC: shape out of range");
-    const size_t smem = series_smem_bytes(dmax, a.nfft, a.nact);
-    rt::raise_smem_limit(mac_series_kernel, smem);
-    const unsigned grid = persistent_grid(mac_series_kernel, SERIES_THREADS, smem, a.nbins);
+    const size_t smem = table_smem_bytes(dmax, a.nfft, TS * groups);
+    rt::raise_smem_limit(mac_table_kernel<TS, TM>, smem);
+    const unsigned nt = (unsigned)(ndt * groups);
+    const unsigned grid = persistent_grid(mac_table_kernel<TS, TM>, nt, smem, a.nbins);
     const int per = (int)((a.nbins + grid - 1) / grid);
-    mac_series_kernel<<<(unsigned)((a.nbins + per - 1) / per), SERIES_THREADS, smem, s>>>(a, dmax, per);
+    mac_table_kernel<TS, TM><<<(unsigned)((a.nbins + per - 1) / per), nt, smem, s>>>(a, dmax, per, ts, groups);
     RT_CHECK(cudaGetLastError());
+}
+
+template <int TS>
+void launch_mac_table_dms(const MacArgs& a, int dmax, int tm, int ts, int ndt, int groups, cudaStream_t s)
+{
+    switch (tm) {
+    case 8:
+        if constexpr (TS == 1) {
+            launch_mac_table<TS, 8>(a, dmax, ts, ndt, groups, s);
+            break;
+        }
+        [[fallthrough]];
+    case 4: launch_mac_table<TS, 4>(a, dmax, ts, ndt, groups, s); break;
+    case 2: launch_mac_table<TS, 2>(a, dmax, ts, ndt, groups, s); break;
+    default: launch_mac_table<TS, 1>(a, dmax, ts, ndt, groups, s); break;
+    }
+}
+}  // namespace
+
+void launch_fdd_mac_table(const MacArgs& a, int dmax, cudaStream_t s)
+{
+    if (!fdd_mac_table_fits(dmax, a.nfft, a.ndm, a.nact, a.nseg))
+        DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "FP32 table MAC: shape out of range");
+    const TableShape t(a.ndm, a.nseg, dmax);
+    const int tm = t.tm, ts = t.ts, ndt = t.ndt, groups = t.groups;
+    switch (ts) {
+    case 1: launch_mac_table_dms<1>(a, dmax, tm, ts, ndt, groups, s); break;
+    case 2: launch_mac_table_dms<2>(a, dmax, tm, ts, ndt, groups, s); break;
+    case 3: launch_mac_table_dms<3>(a, dmax, tm, ts, ndt, groups, s); break;
+    case 4: launch_mac_table_dms<4>(a, dmax, tm, ts, ndt, groups, s); break;
+    case 5: launch_mac_table_dms<5>(a, dmax, tm, ts, ndt, groups, s); break;
+    case 6: launch_mac_table_dms<6>(a, dmax, tm, ts, ndt, groups, s); break;
+    case 7: launch_mac_table_dms<7>(a, dmax, tm, ts, ndt, groups, s); break;
+    case 8: launch_mac_table_dms<8>(a, dmax, tm, ts, ndt, groups, s); break;
+    case 9: launch_mac_table_dms<9>(a, dmax, tm, ts, ndt, groups, s); break;
+    default: launch_mac_table_dms<10>(a, dmax, tm, ts, ndt, groups, s); break;
+    }
 }
 
 void launch_fdd_mac_plain(const MacArgs& a, cudaStream_t s)
