@@ -73,12 +73,17 @@ constexpr size_t TC_MAX_SMEM = kTcMaxSmem;
 //     columns at 384 and 448: 16 MMAs per chunk instead of 24 (one thread
 //     issues an MMA about every 30 ns whatever its N, so narrow MMAs are
 //     bound by their count).
-template <bool FUSED, bool DEEP = false>
+//   fused wide, two buffers (FUSED and WIDE, npad <= 64; the default for 33 to
+//     64 columns): 2 A buffers (0, 128) leave 256 columns, two accumulators of
+//     2 npad <= 128 at 256 and 384. 1024 channels, 2048 DMs, 16385 bins, MAC ms,
+//     deep form -> here: 33.6 -> 27.8 at npad 48, 35.7 -> 31.8 at 64 (and rel-L2
+//     7.7e-6 -> 5.8e-6: the split products sum apart until the read-out).
+template <bool FUSED, bool DEEP, bool WIDE = false>
 struct TcForm {
-    static constexpr bool NARROW = FUSED && !DEEP;        // fused at 32-channel chunks
+    static constexpr bool NARROW = FUSED && !DEEP && !WIDE;  // fused at 32-channel chunks
     static constexpr int CH = NARROW ? 32 : 64;           // channels per A chunk
     static constexpr int PART_CH = CH / TC_PARTS;         // per producer thread
-    static constexpr int NBUF = (FUSED || DEEP) ? 3 : 2;  // A buffers
+    static constexpr int NBUF = (NARROW || DEEP) ? 3 : 2;  // A buffers
     static constexpr uint32_t A_COLS = 2 * CH;            // hi CH + lo CH columns
     static constexpr uint32_t A_BASE = NARROW ? 320 : 0;
     static constexpr uint32_t C0 = NARROW ? 0 : DEEP ? 384 : 256, C1 = NARROW ? 160 : DEEP ? 448 : 384;
@@ -379,10 +384,10 @@ __device__ __forceinline__ uint2 split_bf16x2(float re, float im)
 // leader's MMA thread issues M = 256 MMAs over both CTAs' tensor memory, each
 // CTA loads half of every B chunk and produces the phasors of its 128 DMs;
 // the leader claims the pair's items and publishes them to both CTAs.
-template <bool FUSED, bool DEEP, bool PAIR>
+template <bool FUSED, bool DEEP, bool PAIR, bool WIDE = false>
 __global__ void __launch_bounds__(TC_THREADS, 1) fdd_mac_tc_kernel(const __grid_constant__ TcParams P)
 {
-    using F = TcForm<FUSED, DEEP>;
+    using F = TcForm<FUSED, DEEP, WIDE>;
     // descriptors and tensor maps live in the parameter bank (constant
     // operands, no registers); the items in global memory
     const TcMacArgs* descs = P.descs;
@@ -1207,12 +1212,15 @@ TcLayout tc_layout(const std::vector<TcMacArgs>& descs, unsigned* err, bool pair
     // 4491 -> 4101 ms of MAC over the first 12 config-3 beams (reference
     // segments), 1077 -> 872 ms for the config-2 whole-series spectrum
     const bool wide = !pair && (fsel == 0 || fsel == 3) && npad <= 32;
-    L.fused = (wide || (!pair && fsel == 1 && npad <= TC_FUSED_MAX_NPAD)) ? 1 : 0;
+    // and with two A buffers (two accumulators of 2 npad columns beside them)
+    // wherever npad <= 64
+    L.wide2 = !pair && (fsel == 0 || fsel == 3) && !wide && npad <= TC_DEEP_MAX_NPAD ? 1 : 0;
+    L.fused = (wide || L.wide2 || (!pair && fsel == 1 && npad <= TC_FUSED_MAX_NPAD)) ? 1 : 0;
     // three A buffers when the accumulators fit in 64 columns (DEDISP_TC_FORM=2
     // keeps two, for comparison); the wide fused form always has three
     L.deep = (wide || (!L.fused && npad <= TC_DEEP_MAX_NPAD && fsel != 2)) ? 1 : 0;
     // a stage: 2 splits x (CH / 64 atoms) x the CTA's B rows x 128 bytes
-    L.stage_bytes = ((L.fused && !L.deep) ? 2u : 4u) * (uint32_t)(pair ? npad / 2 : npad) * 128u;
+    L.stage_bytes = ((L.fused && !L.deep && !L.wide2) ? 2u : 4u) * (uint32_t)(pair ? npad / 2 : npad) * 128u;
     L.table_entries = (uint32_t)((table + 1) & ~(size_t)1);  // keep the float2 tables 16-byte aligned
     L.tw_hi_entries = (uint32_t)((hi + 1) & ~(size_t)1);
     L.nact_pad = descs[0].nact_pad;
@@ -1356,8 +1364,9 @@ void launch_fdd_mac_tc_list(const TcParams& P, cudaStream_t s)
         RT_CHECK(cudaGetLastError());
         return;
     }
-    auto kern = P.layout.fused  ? (P.layout.deep ? fdd_mac_tc_kernel<true, true, false>
-                                                 : fdd_mac_tc_kernel<true, false, false>)
+    auto kern = P.layout.wide2  ? fdd_mac_tc_kernel<true, false, false, true>
+                : P.layout.fused ? (P.layout.deep ? fdd_mac_tc_kernel<true, true, false>
+                                                  : fdd_mac_tc_kernel<true, false, false>)
                 : P.layout.deep ? fdd_mac_tc_kernel<false, true, false>
                                 : fdd_mac_tc_kernel<false, false, false>;
     rt::raise_smem_limit(kern, P.layout.smem_bytes);
@@ -1368,7 +1377,7 @@ void launch_fdd_mac_tc_list(const TcParams& P, cudaStream_t s)
 
 int tc_form_code(const TcLayout& L)
 {
-    return L.fused ? (L.deep ? 5 : 1) : L.pair ? (L.deep ? 4 : 3) : L.deep ? 2 : 0;
+    return L.fused ? (L.deep || L.wide2 ? 5 : 1) : L.pair ? (L.deep ? 4 : 3) : L.deep ? 2 : 0;
 }
 
 int launch_fdd_mac_tc(const TcMacArgs& a, const void* B, void* d_items, size_t items_bytes, cudaStream_t s)
