@@ -360,7 +360,17 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     // than one gulp the input rows and the output rows of a gulp have two
     // buffers each, so that gulp g+1's host-to-device copy and gulp g-1's
     // device-to-host copy run while gulp g is dedispersed.
-    const size_t gulp_default = dev_in && dev_out ? kDefaultGulp : kHostDefaultGulp;
+    size_t gulp_default = dev_in && dev_out ? kDefaultGulp : kHostDefaultGulp;
+    if (!dev_in && !(gulp_set && gulp_size)) {
+        // Pinned buffers: at least eight gulps, so that the input copies, the
+        // kernels and the output copies of a call of up to 2^18 samples overlap
+        // as well (1024 channels, 512 trials, 259522 samples: 16.4 ms in one
+        // gulp, 12.4 in nine), but each at least four times the overlap rows
+        // that it copies again. Pageable copies wait in the driver: no gain.
+        const size_t fine = std::max<size_t>({nsamp_out / 8, 4 * (size_t)s.tmax, 8192});
+        if (fine < std::min(nsamp_out, gulp_default) && rt::is_pinned_host(c.in) && rt::is_pinned_host(c.out))
+            gulp_default = fine;
+    }
     size_t G = std::min(nsamp_out, gulp_set && gulp_size ? gulp_size : gulp_default);
     G = std::min(G, (size_t)65535 * bt);
     if (G < nsamp_out && G > bt) G = G / bt * bt;  // whole time tiles in every gulp but the last
@@ -383,12 +393,22 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
         if (!dev_in) b += nbuf_for(g) * in_bytes_for(g);
         return b;
     };
-    size_t free_b = 0, total_b = 0;
-    RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
-    const size_t avail = free_b + m_tr.capacity() + m_q.capacity() + m_out[0].capacity() + m_out[1].capacity() +
-                         m_stage[0].capacity() + m_stage[1].capacity();
-    while (G > bt && bytes_for(G) > avail / 100 * 90) G = round_up(G / 2, bt);
-    if (bytes_for(G) > avail) DD_THROW(DEDISP_MEM_ALLOC_FAILED);
+    // buffers of an earlier call that are large enough need no look at the
+    // free memory (64 channels, 32 trials, 8126 samples from host memory: 0.21
+    // ms with it and a second wait for the error word, 0.135 without)
+    const size_t nb = nbuf_for(G);
+    const bool held = (quad ? m_q.capacity() >= (v.nchans + 1) * qpitch_for(G) * 4
+                            : m_tr.capacity() >= (v.nchans + 1) * pitch_for(G) * 4) &&
+                      (dev_out || std::min(m_out[0].capacity(), m_out[nb - 1].capacity()) >= ndm * G * ob) &&
+                      (dev_in || std::min(m_stage[0].capacity(), m_stage[nb - 1].capacity()) >= in_bytes_for(G));
+    if (!held) {
+        size_t free_b = 0, total_b = 0;
+        RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
+        const size_t avail = free_b + m_tr.capacity() + m_q.capacity() + m_out[0].capacity() +
+                             m_out[1].capacity() + m_stage[0].capacity() + m_stage[1].capacity();
+        while (G > bt && bytes_for(G) > avail / 100 * 90) G = round_up(G / 2, bt);
+        if (bytes_for(G) > avail) DD_THROW(DEDISP_MEM_ALLOC_FAILED);
+    }
 
     const size_t nbuf = nbuf_for(G);
     const size_t pitch = pitch_for(G);
@@ -406,6 +426,7 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     uint32_t* tr = m_tr.get<uint32_t>();
     if (quad) {
         m_err.reserve(sizeof(unsigned));
+        m_err_host.reserve(sizeof(unsigned));
         RT_CHECK(cudaMemsetAsync(m_err.get(), 0, sizeof(unsigned), ex));
     }
 
@@ -555,9 +576,12 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
 
     const bool async = (c.flags & DEDISP_ASYNC) && dev_in;
     if (!async) {
+        // the error word comes back behind the kernels, before the one wait
+        if (quad)
+            RT_CHECK(cudaMemcpyAsync(m_err_host.get(), m_err.get(), sizeof(unsigned), cudaMemcpyDeviceToHost, ex));
         RT_CHECK(cudaStreamSynchronize(ex));
         if (!dev_out) RT_CHECK(cudaStreamSynchronize(d2h));
-        if (quad && kern::read_error_word(m_err.get<unsigned>(), ex))
+        if (quad && *m_err_host.get<unsigned>())
             DD_THROW_MSG(DEDISP_INTERNAL_GPU_ERROR, "a staged window copy did not complete");
     }
     if (record_timing) {
