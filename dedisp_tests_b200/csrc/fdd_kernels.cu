@@ -1204,12 +1204,21 @@ __global__ void __launch_bounds__(MAC_THREADS) mac_plain_kernel(MacArgs a, int b
 // and computed each phasor from the twiddle tables. Packed fma.rn.f32x2 was
 // slower (20.1 ms against 14.4 at 9 segments): two moves per FMA to build its
 // operand pairs.
+//
+// MIRROR: bins k and N/2 - k together. exp(2 pi i (N/2 - k) d / N) = (-1)^d
+// conj(exp(2 pi i k d / N)), so one table, delay and load serve both bins, and
+// the second phasor is two sign flips. The 8-byte gathers took 4.4 wavefronts
+// each for bank conflicts and bounded the narrow tiles: 17.9 -> 12.6 ms at one
+// segment, 7.5 -> 6.8 at four; from five on the FMAs bound and it costs (8.4
+// against 8.6).
+//
 // Measured on B200, 1024 channels, ms, tiled (one segment: 8 DMs a thread of 256)
 // -> here: 512 DMs x 16385 bins x 9 segments 74.6 -> 14.4; 2048 DMs x 39 segments
-// 336 -> 255; 512 DMs x 73728 bins x 1 segment 56.7 -> 17.9.
+// 336 -> 255; 512 DMs x 73728 bins x 1 segment 56.7 -> 12.6.
 constexpr int TAB_THREADS = 256;
 constexpr int TAB_CK = 128;      // channels staged at a time
 constexpr int TAB_MAX_TS = 10;
+constexpr int TAB_MIRROR_TS = 4;  // segment tiles up to this take mirrored bins
 
 __device__ __forceinline__ float2 lds_float2(uint32_t addr)
 {
@@ -1218,7 +1227,7 @@ __device__ __forceinline__ float2 lds_float2(uint32_t addr)
     return v;
 }
 
-template <int TS, int TM>
+template <int TS, int TM, bool MIRROR>
 __global__ void __launch_bounds__(TAB_THREADS) mac_table_kernel(MacArgs a, int dmax, int bins_per_block, int ts, int groups)
 {
     extern __shared__ __align__(16) float2 s_tab[];
@@ -1227,7 +1236,8 @@ __global__ void __launch_bounds__(TAB_THREADS) mac_table_kernel(MacArgs a, int d
     float2* table = s_tab;
     float2* lo = table + tab_n;
     float2* hi = lo + 256;
-    const int width = TS * groups;                              // columns staged, ts used of each TS
+    constexpr int SIDES = MIRROR ? 2 : 1;
+    const int half = TS * groups, width = SIDES * half;         // columns staged, ts used of each TS
     float2* xs = hi + ((nhi + 1u) & ~1u);                       // [TAB_CK][width]
     float* dl = reinterpret_cast<float*>(xs + TAB_CK * width);  // [TAB_CK]
     const int tid = threadIdx.x, nt = blockDim.x;
@@ -1240,8 +1250,9 @@ __global__ void __launch_bounds__(TAB_THREADS) mac_table_kernel(MacArgs a, int d
     const uint32_t table_d0 = (uint32_t)__cvta_generic_to_shared(table) - 8u * 0x4B000000u;
 
     const size_t kb0 = (size_t)blockIdx.x * bins_per_block;
-    const size_t kb1 = min(a.nbins, kb0 + bins_per_block);
+    const size_t kb1 = min(MIRROR ? (size_t)a.nfft / 4 + 1 : a.nbins, kb0 + bins_per_block);
     for (size_t k = kb0; k < kb1; ++k) {
+        const size_t k2 = a.nfft / 2 - k;  // the mirrored bin
         __syncthreads();  // the previous bin's table is no longer read
         {
             uint32_t idx = (uint32_t)(((uint64_t)k * (uint64_t)tid) % a.nfft);
@@ -1256,21 +1267,26 @@ __global__ void __launch_bounds__(TAB_THREADS) mac_table_kernel(MacArgs a, int d
             const int ns = min(ts, a.nseg - sg);        // (none: <= 0)
             for (int m0 = 0; m0 < a.ndm; m0 += ndt * TM) {
                 float dmv[TM];
-                float2 acc[TM][TS];
+                float2 acc[SIDES][TM][TS];
 #pragma unroll
                 for (int q = 0; q < TM; ++q) {
                     dmv[q] = a.dms[min(m0 + dt + q * ndt, a.ndm - 1)];
 #pragma unroll
-                    for (int s = 0; s < TS; ++s) acc[q][s] = make_float2(0.f, 0.f);
+                    for (int s = 0; s < TS; ++s)
+#pragma unroll
+                        for (int h = 0; h < SIDES; ++h) acc[h][q][s] = make_float2(0.f, 0.f);
                 }
                 for (int c0 = 0; c0 < a.nact; c0 += TAB_CK) {
                     const int nc = min(TAB_CK, a.nact - c0);
                     __syncthreads();  // the staged channels are no longer read
                     for (int i = tid; i < TAB_CK * width; i += nt) {
                         const int col = i / TAB_CK, c = i - col * TAB_CK;
-                        const int g = col / TS, s = col - g * TS, seg = s0 + g * ts + s;
+                        const bool second = MIRROR && col >= half;
+                        const int hc = second ? col - half : col;
+                        const int g = hc / TS, s = hc - g * TS, seg = s0 + g * ts + s;
                         float2 v = make_float2(0.f, 0.f);
-                        if (s < ts && seg < a.nseg && c < nc) v = a.Xt[(k * a.nseg + seg) * (size_t)a.nact + c0 + c];
+                        if (s < ts && seg < a.nseg && c < nc)
+                            v = a.Xt[((second ? k2 : k) * a.nseg + seg) * (size_t)a.nact + c0 + c];
                         xs[c * width + col] = v;
                     }
                     for (int i = tid; i < nc; i += nt) dl[i] = a.delay_act[c0 + i];
@@ -1279,25 +1295,37 @@ __global__ void __launch_bounds__(TAB_THREADS) mac_table_kernel(MacArgs a, int d
 #pragma unroll 2
                     for (int c = 0; c < nc; ++c, xc += width) {
                         const float delay = dl[c];
-                        float2 av[TM];
+                        float2 av[SIDES][TM];
 #pragma unroll
                         for (int q = 0; q < TM; ++q) {
                             const float x = __fmul_rn(dmv[q], delay);
                             const float y = rn ? __fadd_rn(x, 8388608.0f) : __fadd_rz(x, 8388608.0f);
                             // 2^23 + d: d in the low mantissa bits
-                            av[q] = lds_float2(table_d0 + 8u * __float_as_uint(y));
-                        }
-#pragma unroll
-                        for (int s = 0; s < TS; ++s) {
-                            const float2 b = xc[s];
-#pragma unroll
-                            for (int q = 0; q < TM; ++q) {
-                                acc[q][s].x = fmaf(av[q].x, b.x, acc[q][s].x);
-                                acc[q][s].x = fmaf(-av[q].y, b.y, acc[q][s].x);
-                                acc[q][s].y = fmaf(av[q].x, b.y, acc[q][s].y);
-                                acc[q][s].y = fmaf(av[q].y, b.x, acc[q][s].y);
+                            const uint32_t bits = __float_as_uint(y);
+                            av[0][q] = lds_float2(table_d0 + 8u * bits);
+                            if constexpr (MIRROR) {
+                                // (-1)^d conj
+                                const uint32_t odd = bits << 31;
+                                av[SIDES - 1][q] =
+                                    make_float2(__uint_as_float(__float_as_uint(av[0][q].x) ^ odd),
+                                                __uint_as_float(__float_as_uint(av[0][q].y) ^ odd ^ 0x80000000u));
                             }
                         }
+#pragma unroll
+                        for (int h = 0; h < SIDES; ++h)
+#pragma unroll
+                            for (int s = 0; s < TS; ++s) {
+                                const float2 b = xc[h * half + s];
+#pragma unroll
+                                for (int q = 0; q < TM; ++q) {
+                                    const float2 w = av[h][q];
+                                    float2& y = acc[h][q][s];
+                                    y.x = fmaf(w.x, b.x, y.x);
+                                    y.x = fmaf(-w.y, b.y, y.x);
+                                    y.y = fmaf(w.x, b.y, y.y);
+                                    y.y = fmaf(w.y, b.x, y.y);
+                                }
+                            }
                     }
                 }
 #pragma unroll
@@ -1306,7 +1334,9 @@ __global__ void __launch_bounds__(TAB_THREADS) mac_table_kernel(MacArgs a, int d
                     if (m >= a.ndm) continue;
 #pragma unroll
                     for (int s = 0; s < TS; ++s)
-                        if (s < ns) a.Yt[(k * a.nseg + sg + s) * (size_t)a.ndm + m] = acc[q][s];
+#pragma unroll
+                        for (int h = 0; h < SIDES; ++h)
+                            if (s < ns) a.Yt[((h ? k2 : k) * a.nseg + sg + s) * (size_t)a.ndm + m] = acc[h][q][s];
                 }
             }
         }
@@ -1638,19 +1668,22 @@ bool fdd_mac_table_fits(int dmax, unsigned nfft, int ndm, int nact, int nseg)
     // 18347 delays: 5.3 ms against 7.5)
     if (nseg > TAB_MAX_TS && (long)dmax > (long)ndm * nact) return false;
     const TableShape t(ndm, nseg, dmax);
-    return table_smem_bytes(dmax, nfft, t.ts * t.groups) <= 200 * 1024;
+    return table_smem_bytes(dmax, nfft, (t.ts <= TAB_MIRROR_TS ? 2 : 1) * t.ts * t.groups) <= 200 * 1024;
 }
 
 namespace {
 template <int TS, int TM>
 void launch_mac_table(const MacArgs& a, int dmax, int ts, int ndt, int groups, cudaStream_t s)
 {
-    const size_t smem = table_smem_bytes(dmax, a.nfft, TS * groups);
-    rt::raise_smem_limit(mac_table_kernel<TS, TM>, smem);
+    constexpr bool MIRROR = TS <= TAB_MIRROR_TS;
+    auto kfn = mac_table_kernel<TS, TM, MIRROR>;
+    const size_t smem = table_smem_bytes(dmax, a.nfft, (MIRROR ? 2 : 1) * TS * groups);
+    rt::raise_smem_limit(kfn, smem);
     const unsigned nt = (unsigned)(ndt * groups);
-    const unsigned grid = persistent_grid(mac_table_kernel<TS, TM>, nt, smem, a.nbins);
-    const int per = (int)((a.nbins + grid - 1) / grid);
-    mac_table_kernel<TS, TM><<<(unsigned)((a.nbins + per - 1) / per), nt, smem, s>>>(a, dmax, per, ts, groups);
+    const size_t units = MIRROR ? (size_t)a.nfft / 4 + 1 : a.nbins;
+    const unsigned grid = persistent_grid(kfn, nt, smem, units);
+    const int per = (int)((units + grid - 1) / grid);
+    kfn<<<(unsigned)((units + per - 1) / per), nt, smem, s>>>(a, dmax, per, ts, groups);
     RT_CHECK(cudaGetLastError());
 }
 
