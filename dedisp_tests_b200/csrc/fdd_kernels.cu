@@ -7,9 +7,11 @@
 //                       half-length complex transform
 //   to_binmajor         X[c][seg][k] -> Xt[k][seg][j] (active channels,
 //                       killmask multiplier folded in)
-//   mac_plain           per-bin complex GEMM on CUDA cores: phasors
-//                       W(k*d mod N) generated on chip from exact integer
-//                       phase indices and a two-level twiddle table
+//   mac_table           per-bin complex GEMM on CUDA cores, phasors from a
+//                       table of W(k*d mod N) over the delays of the bin
+//   mac_plain           the same where that table does not fit: phasors
+//                       generated per use from exact integer phase indices
+//                       and a two-level twiddle table
 //   to_dmmajor / spectrum_out
 //
 // Conventions follow the reference: forward transform e^{-2 pi i k n/N}
@@ -618,9 +620,9 @@ void launch_c2r_4step(float2* Y, size_t bin_pitch, size_t rows, size_t nseg, flo
 // n = n1 + P n2 and k = Q k1 + k2,
 //   Z[Q k1 + k2] = sum_n1 W_P^{n1 k1} W_M^{n1 k2} sum_n2 z[n1 + P n2] W_Q^{n2 k2}:
 // (1) Q-point DFTs over n2 for tiles of T consecutive n1 (mixed-radix
-//     Stockham passes in shared memory; radices 4, 2, 3, 5, 7 in registers,
-//     larger prime radices as direct sums), times W_M^{n1 k2}, stored as rows
-//     k2 of P points in scratch;
+//     Stockham passes; radices up to 16 in registers, prime radices above as
+//     direct sums), times W_M^{n1 k2}, stored as rows k2 of P points in
+//     scratch;
 // (2) P-point transforms of those rows (the shared-memory radix-16 kernel).
 // The spectrum stays in this transposed order: bin k < M of a row at position
 // (k mod Q) P + k / Q, bin M at position M (BinMap); the layout kernels read
@@ -632,104 +634,200 @@ void launch_c2r_4step(float2* Y, size_t bin_pitch, size_t rows, size_t nseg, flo
 constexpr int FQ_LOGP = 13;
 constexpr unsigned FQ_P = 1u << FQ_LOGP;
 constexpr int FQ_THREADS = 256;
+constexpr int FQ_CTAS = 2;     // per SM
+constexpr int FQ_MAX_R = 16;   // largest radix done in registers
 
-// One radix-r pass over T columns of Q points ([T][Q] in shared memory,
-// from `in` to `out`); Ns = product of the earlier passes' radices;
-// wq[x] = W_Q^x (conjugated for the inverse).
-template <bool INV>
-__device__ __forceinline__ void stockham_pass(const float2* __restrict__ in, float2* __restrict__ out, int Q,
-                                              int T, int r, int Ns, const float2* __restrict__ wq)
+// cos and sin of 2 pi x / R for 0 <= x < R at compile time: Taylor series of
+// the angle brought into [-pi, pi], 40 terms (the last below 1e-24).
+__host__ __device__ constexpr double turn_cos(int x, int R)
 {
-    const int R = Q / r;
-    const int ws = Q / (Ns * r);  // W_{Ns r}^x = W_Q^{x ws}
-    const int wr = R;             // W_r^x = W_Q^{x Q / r}
-    auto W = [&](int x) {
-        const float2 w = wq[x];
-        return INV ? conjf2(w) : w;
-    };
-    if (r <= 8) {
-        for (int g = threadIdx.x; g < T * R; g += blockDim.x) {
-            const int col = g / R, j = g - col * R;
-            const int k = j % Ns;
-            const float2* src = in + col * Q + j;
-            float2 v[8];
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                if (t < r) {
-                    float2 a = src[t * R];
-                    if (t > 0 && k > 0) a = cmul(a, W(t * k * ws));
-                    v[t] = a;
-                }
-            }
-            float2* dst = out + col * Q + (j / Ns) * Ns * r + k;
-            if (r == 2) {
-                dst[0] = v[0] + v[1];
-                dst[Ns] = v[0] - v[1];
-            } else if (r == 4) {
-                const float2 s02 = v[0] + v[2], d02 = v[0] - v[2], s13 = v[1] + v[3], d13 = v[1] - v[3];
-                // W_4 = -i (forward) or +i (inverse) times d13
-                const float2 rot = INV ? make_float2(-d13.y, d13.x) : make_float2(d13.y, -d13.x);
-                dst[0] = s02 + s13;
-                dst[Ns] = d02 + rot;
-                dst[2 * Ns] = s02 - s13;
-                dst[3 * Ns] = d02 - rot;
-            } else {
-                // W_r^{t u} = W_Q^{t u wr}: index stepped by u wr (mod Q)
-                for (int u = 0; u < r; ++u) {
-                    float2 acc = v[0];
-                    const int su = u * wr;
-                    int x = 0;
-#pragma unroll
-                    for (int t = 1; t < 8; ++t) {
-                        if (t < r) {
-                            x += su;
-                            if (x >= Q) x -= Q;
-                            acc = acc + cmul(v[t], W(x));
-                        }
-                    }
-                    dst[u * Ns] = acc;
-                }
-            }
+    const double a = 2.0 * 3.14159265358979323846 * (double)(2 * x > R ? x - R : x) / (double)R;
+    double term = 1.0, sum = 1.0;
+    for (int i = 1; i <= 20; ++i) {
+        term *= -a * a / (double)((2 * i - 1) * (2 * i));
+        sum += term;
+    }
+    return sum;
+}
+__host__ __device__ constexpr double turn_sin(int x, int R)
+{
+    const double a = 2.0 * 3.14159265358979323846 * (double)(2 * x > R ? x - R : x) / (double)R;
+    double term = a, sum = a;
+    for (int i = 1; i <= 20; ++i) {
+        term *= -a * a / (double)((2 * i) * (2 * i + 1));
+        sum += term;
+    }
+    return sum;
+}
+
+// W_R^x = exp(-2 pi i x / R).
+template <int R>
+struct Roots {
+    float c[R], s[R];
+    __host__ __device__ constexpr Roots() : c(), s()
+    {
+        for (int x = 0; x < R; ++x) {
+            c[x] = (float)turn_cos(x, R);
+            s[x] = (float)-turn_sin(x, R);
         }
+    }
+};
+
+// R-point DFT, R = 2, 4 or an odd prime, in place. Odd primes pair the inputs
+// t and R - t: half the multiplications of the direct sum.
+template <int R, bool INV>
+__device__ __forceinline__ void dft_prime(float2 (&v)[R])
+{
+    if constexpr (R == 2) {
+        const float2 a = v[0], b = v[1];
+        v[0] = a + b;
+        v[1] = a - b;
+    } else if constexpr (R == 4) {
+        const float2 s02 = v[0] + v[2], d02 = v[0] - v[2], s13 = v[1] + v[3], d13 = v[1] - v[3];
+        // W_4 = -i (forward) or +i (inverse) times d13
+        const float2 rot = INV ? make_float2(-d13.y, d13.x) : make_float2(d13.y, -d13.x);
+        v[0] = s02 + s13;
+        v[1] = d02 + rot;
+        v[2] = s02 - s13;
+        v[3] = d02 - rot;
     } else {
-        // one output (butterfly j, output u) per work item
-        for (int g = threadIdx.x; g < T * Q; g += blockDim.x) {
-            const int col = g / Q, rem = g - col * Q;
-            const int j = rem % R, u = rem / R;
-            const int k = j % Ns;
-            const float2* src = in + col * Q + j;
-            float2 acc = src[0];
-            // input twiddle W_{Ns r}^{t k} times W_r^{t u}: W_Q^{t s}, s = k ws + u wr
-            // (wr r = Q), the index stepped by s (mod Q)
-            const int s = (k * ws + u * wr) % Q;
-            int x = 0;
-            for (int t = 1; t < r; ++t) {
-                x += s;
-                if (x >= Q) x -= Q;
-                acc = acc + cmul(src[t * R], W(x));
+        constexpr Roots<R> w;
+        constexpr int H = (R - 1) / 2;
+        float2 s[H], d[H];
+#pragma unroll
+        for (int t = 0; t < H; ++t) {
+            s[t] = v[t + 1] + v[R - 1 - t];
+            d[t] = v[t + 1] - v[R - 1 - t];
+        }
+        const float2 v0 = v[0];
+        float2 sum = v0;
+#pragma unroll
+        for (int t = 0; t < H; ++t) sum = sum + s[t];
+        v[0] = sum;
+#pragma unroll
+        for (int u = 1; u <= H; ++u) {
+            float2 a = v0, b = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int t = 0; t < H; ++t) {
+                const float c = w.c[((t + 1) * u) % R], n = w.s[((t + 1) * u) % R];
+                a.x += s[t].x * c;
+                a.y += s[t].y * c;
+                b.x += d[t].x * n;
+                b.y += d[t].y * n;
             }
-            out[col * Q + (j / Ns) * Ns * r + k + u * Ns] = acc;
+            // i b forward (w.s holds -sin), -i b for the inverse
+            const float2 ib = INV ? make_float2(b.y, -b.x) : make_float2(-b.y, b.x);
+            v[u] = a + ib;
+            v[R - u] = a - ib;
         }
     }
 }
 
-// All passes; returns the buffer holding the natural-order result.
-template <bool INV>
-__device__ __forceinline__ float2* stockham_all(float2* b0, float2* b1, int Q, int T, const QRadices& rad,
-                                                const float2* wq)
+// R-point DFT of registers, R = 2..16, natural order: Stockham passes of
+// radices 4, 2 and odd primes with every index and root a constant.
+template <int R, int NS, bool INV>
+__device__ __forceinline__ void dft_steps(float2 (&v)[R])
 {
-    float2* cur = b0;
-    float2* nxt = b1;
-    int Ns = 1;
-    for (int p = 0; p < rad.n; ++p) {
-        stockham_pass<INV>(cur, nxt, Q, T, rad.r[p], Ns, wq);
-        __syncthreads();
-        float2* t = cur;
-        cur = nxt;
-        nxt = t;
-        Ns *= rad.r[p];
+    if constexpr (NS < R) {
+        constexpr int L = R / NS;
+        constexpr int r = L % 4 == 0 ? 4 : L % 2 == 0 ? 2 : L % 3 == 0 ? 3 : L % 5 == 0 ? 5 : L;
+        constexpr int J = R / r;
+        constexpr Roots<R> w;
+        float2 o[R];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int k = j % NS;
+            float2 a[r];
+#pragma unroll
+            for (int t = 0; t < r; ++t) {
+                const int x = t * k * (R / (NS * r));
+                a[t] = v[t * J + j];
+                if (x > 0) a[t] = cmul(a[t], make_float2(w.c[x], INV ? -w.s[x] : w.s[x]));
+            }
+            dft_prime<r, INV>(a);
+#pragma unroll
+            for (int u = 0; u < r; ++u) o[(j / NS) * NS * r + k + u * NS] = a[u];
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i) v[i] = o[i];
+        dft_steps<R, NS * r, INV>(v);
     }
-    return cur;
+}
+
+// One radix-R pass over the T = 1 << lt columns of a tile: butterfly j of
+// column col takes the elements t Q/R + j and gives j / Ns * Ns R + j % Ns +
+// u Ns. Consecutive threads hold consecutive columns, so j and all that
+// follows from it is the same over a warp (T >= 32).
+template <int R, bool INV, class Load, class Store>
+__device__ __forceinline__ void q_pass(int Q, int lt, int Ns, const float2* wq, const Load& load, const Store& store)
+{
+    const int J = Q / R, ws = J / Ns;  // W_{Ns R}^x = W_Q^{x ws}
+    for (int g = threadIdx.x; g < J << lt; g += FQ_THREADS) {
+        const int col = g & ((1 << lt) - 1), j = g >> lt;
+        const int b = j / Ns, k = j - b * Ns;
+        float2 v[R];
+#pragma unroll
+        for (int t = 0; t < R; ++t) v[t] = load(col, t * J + j);
+        if (k > 0) {
+#pragma unroll
+            for (int t = 1; t < R; ++t) {
+                const float2 w = wq[t * k * ws];
+                v[t] = cmul(v[t], INV ? conjf2(w) : w);
+            }
+        }
+        dft_steps<R, 1, INV>(v);
+#pragma unroll
+        for (int u = 0; u < R; ++u) store(col, b * Ns * R + k + u * Ns, v[u]);
+    }
+}
+
+// The pass for a prime radix above 16: one output (butterfly j, output u) per
+// work item as a direct sum.
+template <bool INV, class Load, class Store>
+__device__ __forceinline__ void q_pass_direct(int Q, int lt, int r, int Ns, const float2* wq, const Load& load,
+                                              const Store& store)
+{
+    const int J = Q / r, ws = J / Ns;
+    for (int g = threadIdx.x; g < Q << lt; g += FQ_THREADS) {
+        const int col = g & ((1 << lt) - 1), rem = g >> lt;
+        const int u = rem / J, j = rem - u * J;
+        const int b = j / Ns, k = j - b * Ns;
+        float2 acc = load(col, j);
+        // input twiddle W_{Ns r}^{t k} times W_r^{t u}: W_Q^{t s},
+        // s = k ws + u J, the index stepped by s (mod Q)
+        const int s = (k * ws + u * J) % Q;
+        int x = 0;
+        for (int t = 1; t < r; ++t) {
+            x += s;
+            if (x >= Q) x -= Q;
+            acc = acc + cmul(load(col, t * J + j), INV ? conjf2(wq[x]) : wq[x]);
+        }
+        store(col, b * Ns * r + k + u * Ns, acc);
+    }
+}
+
+template <bool INV, class Load, class Store>
+__device__ __forceinline__ void q_pass_any(int r, int Q, int lt, int Ns, const float2* wq, const Load& load,
+                                           const Store& store)
+{
+    switch (r) {
+    case 2: q_pass<2, INV>(Q, lt, Ns, wq, load, store); break;
+    case 3: q_pass<3, INV>(Q, lt, Ns, wq, load, store); break;
+    case 4: q_pass<4, INV>(Q, lt, Ns, wq, load, store); break;
+    case 5: q_pass<5, INV>(Q, lt, Ns, wq, load, store); break;
+    case 6: q_pass<6, INV>(Q, lt, Ns, wq, load, store); break;
+    case 7: q_pass<7, INV>(Q, lt, Ns, wq, load, store); break;
+    case 8: q_pass<8, INV>(Q, lt, Ns, wq, load, store); break;
+    case 9: q_pass<9, INV>(Q, lt, Ns, wq, load, store); break;
+    case 10: q_pass<10, INV>(Q, lt, Ns, wq, load, store); break;
+    case 11: q_pass<11, INV>(Q, lt, Ns, wq, load, store); break;
+    case 12: q_pass<12, INV>(Q, lt, Ns, wq, load, store); break;
+    case 13: q_pass<13, INV>(Q, lt, Ns, wq, load, store); break;
+    case 14: q_pass<14, INV>(Q, lt, Ns, wq, load, store); break;
+    case 15: q_pass<15, INV>(Q, lt, Ns, wq, load, store); break;
+    case 16: q_pass<16, INV>(Q, lt, Ns, wq, load, store); break;
+    default: q_pass_direct<INV>(Q, lt, r, Ns, wq, load, store); break;
+    }
 }
 
 // W_N^t from the two-level table in global memory (L1/L2 resident).
@@ -739,73 +837,139 @@ __device__ __forceinline__ float2 twiddle_g(const TwiddleTable& tw, size_t t, bo
     return inv ? conjf2(w) : w;
 }
 
+// All passes over a tile: the first one takes its elements from `load` and
+// the last one hands them to `store`; those between go through the buffers
+// b0 and b1 ([Q][T], free of bank conflicts). A first pass that reads its
+// elements more than once (the direct sums) finds them staged in b0. At
+// Q = 1 elements only move.
+template <bool INV, class Load, class Store>
+__device__ __forceinline__ void q_transform(int Q, int lt, const QRadices& rad, float2* b0, float2* b1,
+                                            const float2* wq, const Load& load, const Store& store)
+{
+    const int n = Q << lt;
+    if (rad.n == 0) {
+        for (int g = threadIdx.x; g < n; g += FQ_THREADS) store(g, 0, load(g, 0));
+        return;
+    }
+    const bool staged = rad.r[0] > FQ_MAX_R;
+    if (staged) {
+        for (int g = threadIdx.x; g < n; g += FQ_THREADS) b0[g] = load(g & ((1 << lt) - 1), g >> lt);
+    }
+    __syncthreads();  // wq, b0
+    auto from = [&](const float2* s) { return [s, lt](int col, int i) { return s[(i << lt) + col]; }; };
+    auto to = [&](float2* d) { return [d, lt](int col, int i, float2 z) { d[(i << lt) + col] = z; }; };
+    if (rad.n == 1) {
+        if (staged)
+            q_pass_direct<INV>(Q, lt, Q, 1, wq, from(b0), store);
+        else
+            q_pass_any<INV>(Q, Q, lt, 1, wq, load, store);
+        return;
+    }
+    float2* cur = b0;
+    float2* nxt = b1;
+    if (staged) {
+        q_pass_direct<INV>(Q, lt, rad.r[0], 1, wq, from(cur), to(nxt));
+        cur = b1;
+        nxt = b0;
+    } else {
+        q_pass_any<INV>(rad.r[0], Q, lt, 1, wq, load, to(cur));
+    }
+    __syncthreads();
+    int Ns = rad.r[0];
+    for (int p = 1; p + 1 < rad.n; ++p) {
+        q_pass_any<INV>(rad.r[p], Q, lt, Ns, wq, from(cur), to(nxt));
+        __syncthreads();
+        Ns *= rad.r[p];
+        float2* t = cur;
+        cur = nxt;
+        nxt = t;
+    }
+    q_pass_any<INV>(rad.r[rad.n - 1], Q, lt, Ns, wq, from(cur), store);
+}
+
 // Step (1), forward: row `row` = (c, seg) of real samples, columns
 // n1 in [blockIdx.x T, +T): Z1[row][k2 P + n1] = W_M^{n1 k2} DFT_Q(z[n1 + P n2]).
-__global__ void __launch_bounds__(FQ_THREADS) fftq_cols_fwd_kernel(
-    const float* x, size_t x_pitch, size_t nseg, size_t seg_stride, float2* Z1, int Q, int T, QRadices rad,
+//
+// Bound by memory (every point in and out once). A thread keeps a whole
+// butterfly of up to 16 points in registers, all of them at Q <= 16, with its
+// inner indices and roots constants of the code; consecutive threads take
+// consecutive columns, so loads and stores are 256 bytes a warp, the index
+// divisions are uniform, and passes past the first trade through [Q][T]
+// buffers without bank conflicts. One radix-4/3/2 pass at a time through
+// shared memory, with run-time radices and columns as the slow index, cost
+// 3.39 ms for 1024 rows at Q = 9; this form takes 0.325 (3.7 TB/s, 0.56 of
+// a 6.65 TB/s copy). Whole calls of 32 channels and 32 trials: Q = 3
+// 0.86 -> 0.12 ms, 17 4.0 -> 0.47, 65 15.1 -> 2.3, 289 108 -> 39 (with the
+// inverse and the MAC).
+__global__ void __launch_bounds__(FQ_THREADS, FQ_CTAS) fftq_cols_fwd_kernel(
+    const float* x, size_t x_pitch, size_t nseg, size_t seg_stride, float2* Z1, int Q, int lt, int bufs, QRadices rad,
     const float2* wq_g, TwiddleTable tw)
 {
     extern __shared__ __align__(16) float2 s_q[];
-    float2* b0 = s_q;
-    float2* b1 = b0 + T * Q;
-    float2* wq = b1 + T * Q;
-    for (int i = threadIdx.x; i < Q; i += blockDim.x) wq[i] = wq_g[i];
+    float2* wq = s_q;
+    float2* b0 = wq + Q;
+    float2* b1 = bufs > 1 ? b0 + ((size_t)Q << lt) : b0;
+    if (rad.n > 1 || rad.r[0] > FQ_MAX_R)
+        for (int i = threadIdx.x; i < Q; i += FQ_THREADS) wq[i] = wq_g[i];
     const size_t row = blockIdx.y;
-    const unsigned n1_0 = blockIdx.x * (unsigned)T;
+    const unsigned n1_0 = blockIdx.x << lt;
     const size_t c = row / nseg, seg = row - c * nseg;
     const float* xr = x + c * x_pitch + seg * seg_stride;
-    for (int idx = threadIdx.x; idx < T * Q; idx += blockDim.x) {
-        const int col = idx % T, n2 = idx / T;
-        const size_t n = (size_t)n1_0 + col + (size_t)FQ_P * n2;
-        b0[col * Q + n2] = make_float2(xr[2 * n], xr[2 * n + 1]);
-    }
-    __syncthreads();
-    const float2* res = stockham_all<false>(b0, b1, Q, T, rad, wq);
-    const size_t M = (size_t)FQ_P * Q;
-    float2* zo = Z1 + row * M;
-    for (int idx = threadIdx.x; idx < T * Q; idx += blockDim.x) {
-        const int col = idx % T, k2 = idx / T;
-        const size_t n1 = (size_t)n1_0 + col;
-        // W_M^{n1 k2} = W_N^{2 n1 k2}, 2 n1 k2 < 2M = N
-        zo[(size_t)k2 * FQ_P + n1] = cmul(res[col * Q + k2], twiddle_g(tw, 2 * n1 * (size_t)k2, false));
-    }
+    const bool pairs = ((uintptr_t)xr & 7) == 0;
+    float2* zo = Z1 + row * ((size_t)FQ_P * Q);
+    q_transform<false>(
+        Q, lt, rad, b0, b1, wq,
+        [=](int col, int n2) {
+            const size_t n = (size_t)(n1_0 + (unsigned)col) + (size_t)FQ_P * n2;
+            return pairs ? __ldcs((const float2*)xr + n) : make_float2(xr[2 * n], xr[2 * n + 1]);
+        },
+        [=](int col, int k2, float2 z) {
+            const size_t n1 = n1_0 + (unsigned)col;
+            // W_M^{n1 k2} = W_N^{2 n1 k2}, 2 n1 k2 < 2M = N
+            zo[(size_t)k2 * FQ_P + n1] = k2 ? cmul(z, twiddle_g(tw, 2 * n1 * (size_t)k2, false)) : z;
+        });
 }
 
 // Step (1) backwards: u rows k2 (Z1[row][k2 P + n1]) times W_M^{-n1 k2},
 // inverse Q-point DFTs over k2, then z[n1 + P n2] / M as real samples
 // 2n, 2n + 1 of segment `seg` (the first `keep`, at most out_len).
-__global__ void __launch_bounds__(FQ_THREADS) fftq_cols_inv_kernel(
-    const float2* Z1, float* out, size_t out_stride, size_t nseg, size_t keep, size_t out_len, int Q, int T,
-    QRadices rad, const float2* wq_g, TwiddleTable tw)
+__global__ void __launch_bounds__(FQ_THREADS, FQ_CTAS) fftq_cols_inv_kernel(
+    const float2* Z1, float* out, size_t out_stride, size_t nseg, size_t keep, size_t out_len, int Q, int lt,
+    int bufs, QRadices rad, const float2* wq_g, TwiddleTable tw)
 {
     extern __shared__ __align__(16) float2 s_q[];
-    float2* b0 = s_q;
-    float2* b1 = b0 + T * Q;
-    float2* wq = b1 + T * Q;
-    for (int i = threadIdx.x; i < Q; i += blockDim.x) wq[i] = wq_g[i];
+    float2* wq = s_q;
+    float2* b0 = wq + Q;
+    float2* b1 = bufs > 1 ? b0 + ((size_t)Q << lt) : b0;
+    if (rad.n > 1 || rad.r[0] > FQ_MAX_R)
+        for (int i = threadIdx.x; i < Q; i += FQ_THREADS) wq[i] = wq_g[i];
     const size_t row = blockIdx.y;
-    const unsigned n1_0 = blockIdx.x * (unsigned)T;
+    const unsigned n1_0 = blockIdx.x << lt;
     const size_t M = (size_t)FQ_P * Q;
     const float2* zr = Z1 + row * M;
-    for (int idx = threadIdx.x; idx < T * Q; idx += blockDim.x) {
-        const int col = idx % T, k2 = idx / T;
-        const size_t n1 = (size_t)n1_0 + col;
-        b0[col * Q + k2] = cmul(zr[(size_t)k2 * FQ_P + n1], twiddle_g(tw, 2 * n1 * (size_t)k2, true));
-    }
-    __syncthreads();
-    const float2* res = stockham_all<true>(b0, b1, Q, T, rad, wq);
     const float scale = 1.0f / (float)M;
     const size_t dm = row / nseg, seg = row - dm * nseg;
-    float* dst = out + dm * out_stride;
     const size_t o0 = seg * keep;
-    for (int idx = threadIdx.x; idx < T * Q; idx += blockDim.x) {
-        const int col = idx % T, n2 = idx / T;
-        const float2 z = res[col * Q + n2];
-        const size_t n = (size_t)n1_0 + col + (size_t)FQ_P * n2;
-        const size_t i0 = 2 * n, i1 = i0 + 1;
-        if (i0 < keep && o0 + i0 < out_len) dst[o0 + i0] = z.x * scale;
-        if (i1 < keep && o0 + i1 < out_len) dst[o0 + i1] = z.y * scale;
-    }
+    const size_t most = o0 < out_len ? min(keep, out_len - o0) : 0;  // samples of this segment to write
+    float* dst = out + dm * out_stride + o0;
+    const bool pairs = ((uintptr_t)dst & 7) == 0;
+    q_transform<true>(
+        Q, lt, rad, b0, b1, wq,
+        [=](int col, int k2) {
+            const size_t n1 = n1_0 + (unsigned)col;
+            const float2 z = zr[(size_t)k2 * FQ_P + n1];
+            return k2 ? cmul(z, twiddle_g(tw, 2 * n1 * (size_t)k2, true)) : z;
+        },
+        [=](int col, int n2, float2 z) {
+            const size_t i = 2 * ((size_t)(n1_0 + (unsigned)col) + (size_t)FQ_P * n2);
+            const float2 v = make_float2(z.x * scale, z.y * scale);
+            if (pairs && i + 1 < most) {
+                *(float2*)(dst + i) = v;
+            } else {
+                if (i < most) dst[i] = v.x;
+                if (i + 1 < most) dst[i + 1] = v.y;
+            }
+        });
 }
 
 // Step (2): P-point complex transforms of contiguous rows; row g = o Q + k2
@@ -904,13 +1068,35 @@ __global__ void __launch_bounds__(256) c2r_pre_q_kernel(float2* Y, size_t y_pitc
     r[pk] = zk;
 }
 
-// Columns per CTA of step (1): the largest of 16, 8, 4 whose two [T][Q]
-// buffers and the W_Q table fit in shared memory (0: none fits).
-int fftq_tile(unsigned Q)
+// Tile of step (1): columns (1 << lt), buffers and bytes of shared memory.
+struct FqTile {
+    int lt = 2, bufs = 0;
+    size_t smem = 0;
+};
+
+size_t fq_smem(unsigned Q, int lt, int bufs)
 {
-    for (int T : {16, 8, 4})
-        if ((2 * (size_t)T * Q + Q) * sizeof(float2) <= kFqMaxSmem) return T;
-    return 0;
+    return (((size_t)bufs * Q << lt) + Q) * sizeof(float2);
+}
+
+// A length is taken when two buffers of four columns and the W_Q table fit.
+bool fq_fits(unsigned Q)
+{
+    return fq_smem(Q, 2, 2) <= kFqMaxSmem;
+}
+
+// One pass in registers: 256 columns, nothing shared. Otherwise the most
+// columns that leave room for four CTAs an SM, at least a warp's 32 while
+// they fit at all.
+FqTile fq_tile(unsigned Q, const QRadices& rad)
+{
+    FqTile t;
+    const bool staged = rad.n > 0 && rad.r[0] > FQ_MAX_R;
+    t.bufs = std::min(2, std::max(0, rad.n - 1) + (staged ? 1 : 0));
+    for (t.lt = 8; t.lt > 5 && fq_smem(Q, t.lt, t.bufs) > 56 * 1024; --t.lt) {}
+    for (; t.lt > 2 && fq_smem(Q, t.lt, t.bufs) > kFqMaxSmem; --t.lt) {}
+    t.smem = fq_smem(Q, t.lt, t.bufs);
+    return t;
 }
 
 // ---------------------------------------------------------------------------
@@ -1512,7 +1698,7 @@ void make_twiddle_tables(size_t n, std::vector<float2>& lo, std::vector<float2>&
 
 bool fftq_length(size_t nfft)
 {
-    return nfft >= 16384 && nfft % 16384 == 0 && fftq_tile((unsigned)(nfft / 16384)) > 0 &&
+    return nfft >= 16384 && nfft % 16384 == 0 && fq_fits((unsigned)(nfft / 16384)) &&
            nfft / 2 <= ((size_t)1 << 31);
 }
 
@@ -1529,16 +1715,33 @@ BinMap fdd_binmap(size_t nfft)
 QRadices fftq_radices(unsigned Q)
 {
     QRadices r;
-    unsigned q = Q;
     auto push = [&](unsigned f) {
         if (r.n >= 24) DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "too many FFT radices");
         r.r[r.n++] = (int)f;
-        q /= f;
     };
-    for (unsigned f : {4u, 2u, 3u, 5u, 7u})
-        while (q % f == 0) push(f);
-    for (unsigned f = 11; q > 1; f += 2)
-        while (q % f == 0) push(f);
+    // the part with prime factors up to 13, in as few radices up to 16 as it takes
+    unsigned small = 1, rest = Q;
+    for (unsigned f : {2u, 3u, 5u, 7u, 11u, 13u})
+        for (; rest % f == 0; rest /= f) small *= f;
+    auto biggest = [](unsigned q) {  // largest divisor up to FQ_MAX_R
+        unsigned d = std::min(q, (unsigned)FQ_MAX_R);
+        while (q % d) --d;
+        return d;
+    };
+    while (small > 1) {
+        unsigned f = biggest(small);
+        // the last two radices of near-equal size
+        if (small > f && small / f <= (unsigned)FQ_MAX_R)
+            for (unsigned d = small / f; d <= f; ++d)
+                if (small % d == 0 && small / d <= (unsigned)FQ_MAX_R && d >= small / d) {
+                    f = d;
+                    break;
+                }
+        push(f);
+        small /= f;
+    }
+    for (unsigned f = 17; rest > 1; f += 2)
+        for (; rest % f == 0; rest /= f) push(f);
     return r;
 }
 
@@ -1559,11 +1762,10 @@ void launch_fft_r2c_q(const float* x, size_t x_pitch, size_t nchans, size_t nseg
     if (!fftq_length(nfft)) DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "unsupported FFT length");
     const unsigned Q = (unsigned)(nfft / 16384);
     if (nchans * nseg == 0) return;
-    const int T = fftq_tile(Q);
     const QRadices rad = fftq_radices(Q);
+    const FqTile tile = fq_tile(Q, rad);
     const BinMap map = fdd_binmap(nfft);
-    const size_t sq = (2 * (size_t)T * Q + Q) * sizeof(float2);
-    rt::raise_smem_limit(fftq_cols_fwd_kernel, sq);
+    rt::raise_smem_limit(fftq_cols_fwd_kernel, tile.smem);
     auto kr = fft_c2c_rows_kernel<FQ_LOGP, false>;
     const size_t sr = (FQ_P + 256 + 2 * FQ_P / 256) * sizeof(float2);
     rt::raise_smem_limit(kr, sr);
@@ -1572,8 +1774,8 @@ void launch_fft_r2c_q(const float* x, size_t x_pitch, size_t nchans, size_t nseg
         const size_t rows = std::min(per, nchans - c0) * nseg;
         const float* xc = x + c0 * x_pitch;
         float2* Xc = X + c0 * nseg * bin_pitch;
-        fftq_cols_fwd_kernel<<<dim3(FQ_P / T, (unsigned)rows), FQ_THREADS, sq, s>>>(xc, x_pitch, nseg, seg_stride,
-                                                                                  scratch, (int)Q, T, rad, wq, tw);
+        fftq_cols_fwd_kernel<<<dim3(FQ_P >> tile.lt, (unsigned)rows), FQ_THREADS, tile.smem, s>>>(
+            xc, x_pitch, nseg, seg_stride, scratch, (int)Q, tile.lt, tile.bufs, rad, wq, tw);
         RT_CHECK(cudaGetLastError());
         const size_t nrows = rows * Q;
         kr<<<persistent_grid(kr, FftPlan<FQ_LOGP>::threads(), sr, nrows), FftPlan<FQ_LOGP>::threads(), sr, s>>>(
@@ -1592,14 +1794,13 @@ void launch_fft_c2r_q(float2* Y, size_t bin_pitch, size_t ndm, size_t nseg, size
     if (!fftq_length(nfft)) DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "unsupported FFT length");
     const unsigned Q = (unsigned)(nfft / 16384);
     if (ndm * nseg == 0) return;
-    const int T = fftq_tile(Q);
     const QRadices rad = fftq_radices(Q);
+    const FqTile tile = fq_tile(Q, rad);
     const BinMap map = fdd_binmap(nfft);
     auto kr = fft_c2c_rows_kernel<FQ_LOGP, true>;
     const size_t sr = (FQ_P + 256 + 2 * FQ_P / 256) * sizeof(float2);
     rt::raise_smem_limit(kr, sr);
-    const size_t sq = (2 * (size_t)T * Q + Q) * sizeof(float2);
-    rt::raise_smem_limit(fftq_cols_inv_kernel, sq);
+    rt::raise_smem_limit(fftq_cols_inv_kernel, tile.smem);
     const size_t per = rows_per_launch(nseg);
     for (size_t d0 = 0; d0 < ndm; d0 += per) {
         const size_t rows = std::min(per, ndm - d0) * nseg;
@@ -1612,8 +1813,8 @@ void launch_fft_c2r_q(float2* Y, size_t bin_pitch, size_t ndm, size_t nseg, size
         kr<<<persistent_grid(kr, FftPlan<FQ_LOGP>::threads(), sr, nrows), FftPlan<FQ_LOGP>::threads(), sr, s>>>(
             Yd, bin_pitch, scratch, map.M, Q, twp, nrows);
         RT_CHECK(cudaGetLastError());
-        fftq_cols_inv_kernel<<<dim3(FQ_P / T, (unsigned)rows), FQ_THREADS, sq, s>>>(
-            scratch, od, out_stride, nseg, keep, out_len, (int)Q, T, rad, wq, tw);
+        fftq_cols_inv_kernel<<<dim3(FQ_P >> tile.lt, (unsigned)rows), FQ_THREADS, tile.smem, s>>>(
+            scratch, od, out_stride, nseg, keep, out_len, (int)Q, tile.lt, tile.bufs, rad, wq, tw);
         RT_CHECK(cudaGetLastError());
     }
 }
