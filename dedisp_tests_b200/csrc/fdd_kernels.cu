@@ -1869,7 +1869,9 @@ bool fdd_mac_table_fits(int dmax, unsigned nfft, int ndm, int nact, int nseg)
     // 18347 delays: 5.3 ms against 7.5)
     if (nseg > TAB_MAX_TS && (long)dmax > (long)ndm * nact) return false;
     const TableShape t(ndm, nseg, dmax);
-    return table_smem_bytes(dmax, nfft, (t.ts <= TAB_MIRROR_TS ? 2 : 1) * t.ts * t.groups) <= 200 * 1024;
+    // 200 KB for the tables of one segment (lengths up to 6.4 million samples
+    // at small delays, more than the tiled kernel takes) and its staged columns
+    return table_smem_bytes(dmax, nfft, (t.ts <= TAB_MIRROR_TS ? 2 : 1) * t.ts * t.groups) <= 204 * 1024;
 }
 
 namespace {

@@ -34,3 +34,24 @@ def test_segments_and_trials(nseg, ndm, nchans, dm_max, rounding):
     ref = po.fdd_timeseries(x, _delays(params), np.ones(nchans, np.int32), dms, nout, round_delays=int(rounding))
     rel, mx = _errs(out, ref)
     assert rel < FP32_REL_L2 and mx < FP32_MAX_ABS, (rel, mx)
+
+
+def test_longest_series():
+    """N = 16384 x 394, the longest whole series that FP32 plans take (8
+    channels, delays of a few samples; 200 KB of phasor tables). Tolerance as
+    above: the MAC sums 8 products, the transforms lose log2(N) / 2 roundings
+    each way and the direct sums of 197 terms sqrt(197) of one pass, about
+    1.5e-6 relative L2."""
+    nchans, q = 8, 394
+    nsamps = 16384 * q - 700
+    inp, params = _input(nchans, nsamps, 91)
+    dms = np.linspace(0, 40, 3, dtype=np.float32)
+    p = _plan(params, dms, segmented=0, timeseries=True, precision=0)
+    nout = nsamps - p.get_max_delay()
+    out = np.zeros((len(dms), nout), np.float32)
+    p.execute(nsamps, inp, 8, out, 32)
+    x = _oracle_x(inp, nsamps, params, 8)
+    ref = po.fdd_timeseries(x, _delays(params), np.ones(nchans, np.int32), dms, nout)
+    rel, mx = _errs(out, ref)
+    print(f"rel-L2 {rel:.3e} max-abs {mx:.3e}")
+    assert rel < FP32_REL_L2 and mx < FP32_MAX_ABS, (rel, mx)
