@@ -316,9 +316,10 @@ void FddBatch::upload()
     }
     if (descs.size() > (size_t)kern::kTcMaxDesc)
         DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "a batch holds at most 48 beam segment groups");
-    // Segment groups of at most 32 MMA columns take the wide fused form, the
-    // others the three-MMA form: a launch for each class present (a launch's
-    // form follows its widest descriptor).
+    // Segment groups of at most 32 MMA columns take the wide fused form with
+    // three A buffers, the others the one with two (up to 64 columns) or the
+    // three-MMA form: a launch for each class present (a launch's form follows
+    // its widest descriptor).
     std::vector<kern::TcMacArgs> cls_descs[2];
     std::vector<const void*> cls_bs[2];
     for (size_t d = 0; d < descs.size(); ++d) {

@@ -10,8 +10,7 @@
 // split B operand of each segment group, then one persistent tensor-core
 // (3xBF16) MAC launch over a work list of (beam segment group, DM tiles, bin
 // range) items of all beams per MMA-form class (segment groups of at most 32
-// MMA columns take the wide fused form, wider ones the three-MMA form: at
-// most two launches), then per beam the DM-major transpose and the
+// MMA columns, and wider ones: at most two launches), then per beam the DM-major transpose and the
 // inverse FFTs straight into the caller's rows. The sequence is captured once
 // into a CUDA graph and replayed. Results equal those of an FDDGPUPlan per
 // beam (segmented, tensor-core precision), which is what the tests check.
@@ -102,7 +101,7 @@ private:
 
     rt::DeviceBuffer m_chan, m_kmv, m_delay_pad, m_err, m_twp_lo, m_twp_hi;
     // MAC launches: one per MMA-form class of the beams' segment groups
-    // (at most 32 columns: the wide fused form; more: the three-MMA form)
+    // (at most 32 columns, and more)
     rt::DeviceBuffer m_items[2], m_cta_ns[2];
     rt::DeviceBuffer m_own_ws;
     void* m_ext_ws = nullptr;

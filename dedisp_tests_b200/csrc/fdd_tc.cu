@@ -64,10 +64,9 @@ constexpr size_t TC_MAX_SMEM = kTcMaxSmem;
 //     adjacent in shared memory), then Al Bh (N = npad) into its first npad
 //     columns; the epilogue adds the two halves. Accumulators of 160 columns at
 //     0 and 160, 32-channel A chunks in 3 buffers of 64 columns at 320, 384, 448.
-//   deep (npad <= 64): the three-MMA form with 3 A buffers (0, 128, 256) and
-//     accumulators of 64 columns at 384 and 448: half again as many phasors
-//     in flight, which is what bounds the MAC when it waits on MMA
-//     completions rather than on the tensor pipe.
+//   deep (pairs at npad <= 64): the three-MMA form with 3 A buffers (0, 128,
+//     256) and accumulators of 64 columns at 384 and 448: half again as many
+//     phasors in flight.
 //   fused wide (FUSED and DEEP, npad <= 32; the default there): the fused form at 64-channel
 //     chunks, 3 A buffers (0, 128, 256) and accumulators of 2 npad <= 64
 //     columns at 384 and 448: 16 MMAs per chunk instead of 24 (one thread
@@ -76,7 +75,7 @@ constexpr size_t TC_MAX_SMEM = kTcMaxSmem;
 //   fused wide, two buffers (FUSED and WIDE, npad <= 64; the default for 33 to
 //     64 columns): 2 A buffers (0, 128) leave 256 columns, two accumulators of
 //     2 npad <= 128 at 256 and 384. 1024 channels, 2048 DMs, 16385 bins, MAC ms,
-//     deep form -> here: 33.6 -> 27.8 at npad 48, 35.7 -> 31.8 at 64 (and rel-L2
+//     three MMAs with 3 A buffers -> here: 33.6 -> 27.8 at npad 48, 35.7 -> 31.8 at 64 (and rel-L2
 //     7.7e-6 -> 5.8e-6: the split products sum apart until the read-out).
 template <bool FUSED, bool DEEP, bool WIDE = false>
 struct TcForm {
@@ -1201,24 +1200,25 @@ TcLayout tc_layout(const std::vector<TcMacArgs>& descs, unsigned* err, bool pair
         if (a.nact_pad != descs[0].nact_pad)
             DD_THROW_MSG(DEDISP_INTERNAL_GPU_ERROR, "tensor-core MAC: descriptors differ in channels");
     }
-    // MMA form: the three-MMA form unless DEDISP_TC_FORM=1 asks for the fused
-    // form (which needs npad <= 80; its 32-channel chunks double the hand-offs
-    // per channel: config 2 41.6 against 40.5 ms), kept selectable
+    // MMA form. Above 64 columns the three-MMA form (npad 80: 40.5 ms against
+    // 41.6 fused at 32-channel chunks, which double the hand-offs per channel;
+    // DEDISP_TC_FORM=1 selects that one up to 80 columns, 2 the three-MMA form
+    // at any width).
     const char* form = std::getenv("DEDISP_TC_FORM");
     L.pair = pair ? 1 : 0;
     const int fsel = form ? std::atoi(form) : 0;
-    // the fused form at 64-channel chunks wherever npad <= 32 (DEDISP_TC_FORM=1
-    // or 2 select the others): 16 MMAs per chunk instead of 24; measured
-    // 4491 -> 4101 ms of MAC over the first 12 config-3 beams (reference
-    // segments), 1077 -> 872 ms for the config-2 whole-series spectrum
+    // the fused form at 64-channel chunks wherever npad <= 32: 16 MMAs per
+    // chunk instead of 24; measured 4491 -> 4101 ms of MAC over twelve beams of
+    // 1536 channels (reference segments), 1077 -> 872 ms for a whole-series
+    // spectrum of 1024 channels
     const bool wide = !pair && (fsel == 0 || fsel == 3) && npad <= 32;
     // and with two A buffers (two accumulators of 2 npad columns beside them)
     // wherever npad <= 64
     L.wide2 = !pair && (fsel == 0 || fsel == 3) && !wide && npad <= TC_DEEP_MAX_NPAD ? 1 : 0;
     L.fused = (wide || L.wide2 || (!pair && fsel == 1 && npad <= TC_FUSED_MAX_NPAD)) ? 1 : 0;
-    // three A buffers when the accumulators fit in 64 columns (DEDISP_TC_FORM=2
-    // keeps two, for comparison); the wide fused form always has three
-    L.deep = (wide || (!L.fused && npad <= TC_DEEP_MAX_NPAD && fsel != 2)) ? 1 : 0;
+    // three A buffers: the wide fused form, and pairs whose accumulators fit in
+    // 64 columns (DEDISP_TC_FORM=2 keeps two, for comparison)
+    L.deep = (wide || (pair && npad <= TC_DEEP_MAX_NPAD && fsel != 2)) ? 1 : 0;
     // a stage: 2 splits x (CH / 64 atoms) x the CTA's B rows x 128 bytes
     L.stage_bytes = ((L.fused && !L.deep && !L.wide2) ? 2u : 4u) * (uint32_t)(pair ? npad / 2 : npad) * 128u;
     L.table_entries = (uint32_t)((table + 1) & ~(size_t)1);  // keep the float2 tables 16-byte aligned
@@ -1367,8 +1367,7 @@ void launch_fdd_mac_tc_list(const TcParams& P, cudaStream_t s)
     auto kern = P.layout.wide2  ? fdd_mac_tc_kernel<true, false, false, true>
                 : P.layout.fused ? (P.layout.deep ? fdd_mac_tc_kernel<true, true, false>
                                                   : fdd_mac_tc_kernel<true, false, false>)
-                : P.layout.deep ? fdd_mac_tc_kernel<false, true, false>
-                                : fdd_mac_tc_kernel<false, false, false>;
+                                 : fdd_mac_tc_kernel<false, false, false>;
     rt::raise_smem_limit(kern, P.layout.smem_bytes);
     const int grid = std::min(P.nitems, tc_sm_count());
     kern<<<grid, TC_THREADS, P.layout.smem_bytes, s>>>(P);
@@ -1377,7 +1376,7 @@ void launch_fdd_mac_tc_list(const TcParams& P, cudaStream_t s)
 
 int tc_form_code(const TcLayout& L)
 {
-    return L.fused ? (L.deep || L.wide2 ? 5 : 1) : L.pair ? (L.deep ? 4 : 3) : L.deep ? 2 : 0;
+    return L.fused ? (L.deep || L.wide2 ? 5 : 1) : L.pair ? (L.deep ? 4 : 3) : 0;
 }
 
 int launch_fdd_mac_tc(const TcMacArgs& a, const void* B, void* d_items, size_t items_bytes, cudaStream_t s)

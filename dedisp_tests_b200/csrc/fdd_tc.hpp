@@ -57,7 +57,7 @@ struct TcWork {
 struct TcLayout {
     int stages;                // B pipeline depth
     int fused;                 // 1: fused MMA form (largest npad <= 80)
-    int deep;                  // 1: three-MMA form with 3 A buffers (largest npad <= 64)
+    int deep;                  // 1: 3 A buffers (wide fused form; pairs at npad <= 64)
     int wide2;               // fused at 64-channel chunks with two A buffers
     int pair;                  // 1: CTA pairs (cta_group::2, M = 256, npad a multiple of 32)
     uint32_t stage_bytes;      // per stage (largest npad)

@@ -3,8 +3,8 @@
 // One call = validate-free execution of a (sub-)range of the DM list over a
 // time series, in gulps of output samples:
 //   host rows --(H2D, pinned or pageable)--> gulp input buffer --K1d-->
-//   quad-strided rows (quad variants; K1: channel-major packed rows for the
-//   others) --K2--> output --(D2H)--> host rows. With several gulps, input and
+//   quad-strided rows (pattern and quad kernels; K1: channel-major packed
+//   rows for the others) --K2--> output --(D2H)--> host rows. With several gulps, input and
 //   output buffers are doubled so that the copies of neighbouring gulps
 //   overlap a gulp's kernels; the last gulp's K2 and D2H run per DM group.
 // With DEDISP_DEVICE_POINTERS the copies disappear and K1d/K1/K2 read/write
