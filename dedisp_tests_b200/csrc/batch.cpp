@@ -213,9 +213,19 @@ void TddBatch::prepare_patterns()
             if (fit == PatternTables::kTooWide) wide = true;
         }
     }
+    // room for all tables and the workspace, else the row-by-row form
+    size_t tables = 0, free_b = 0, total_b = 0;
+    for (auto& t : m_tables) tables += t->bytes();
+    RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
+    m_pattern = true;
+    const size_t ws = m_ext_ws ? 0 : workspace_bytes(), held = m_own_ws.capacity();
+    if (tables > free_b / 4 || (ws > held && ws + tables > free_b + held)) {
+        m_pattern = false;
+        m_tables.clear();
+        return;
+    }
     for (auto& t : m_tables) t->emit(nullptr);
     RT_CHECK(cudaStreamSynchronize(nullptr));
-    m_pattern = true;
 }
 
 void TddBatch::set_shape(const BatchShape& shape)

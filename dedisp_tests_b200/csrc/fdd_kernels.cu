@@ -1396,7 +1396,10 @@ __global__ void __launch_bounds__(MAC_THREADS) mac_plain_kernel(MacArgs a, int b
 // the second phasor is two sign flips. The 8-byte gathers took 4.4 wavefronts
 // each for bank conflicts and bounded the narrow tiles: 17.9 -> 12.6 ms at one
 // segment, 7.5 -> 6.8 at four; from five on the FMAs bound and it costs (8.4
-// against 8.6).
+// against 8.6). Four bins a gather (N/4 -+ k too, i^d by selects) took 13.3 ms
+// at one segment, packed multiply-adds on doubled spectra 13.3 to 14.1: with
+// two bins neither gathers nor issue slots bind alone, the chain from delay to
+// sum does.
 //
 // Measured on B200, 1024 channels, ms, tiled (one segment: 8 DMs a thread of 256)
 // -> here: 512 DMs x 16385 bins x 9 segments 74.6 -> 14.4; 2048 DMs x 39 segments

@@ -105,8 +105,25 @@ PatternTables::Fit PatternTables::fit(cudaStream_t st)
     // samples apart, 2 bits: 0.240 ms here against 0.231 at nearly equal
     // wavefronts; 5% below them the two are even).
     const unsigned long long rows = (unsigned long long)m_args.ndm * m_args.nact * m_args.lane_words;
-    const size_t piece = sizeof(kern::PatternPiece) + 16 * sizeof(uint4) + (size_t)m_total.rec_words * 4;
-    return m_total.cost * 8 < rows * 7 && m_total.pieces * piece <= ((size_t)2 << 30) ? kUse : kRowsFaster;
+    if (m_total.cost * 8 >= rows * 7 || bytes() > ((size_t)2 << 30)) return kRowsFaster;
+    if (bytes() > m_tables.capacity()) {
+        // where memory is scarce it is left to the rows and outputs
+        size_t free_b = 0, total_b = 0;
+        RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
+        if (bytes() > (free_b + m_tables.capacity()) / 4) return kRowsFaster;
+    }
+    return kUse;
+}
+
+size_t PatternTables::bytes() const
+{
+    return m_total.pieces * (sizeof(kern::PatternPiece) + 16 * sizeof(uint4) + (size_t)m_total.rec_words * 4);
+}
+
+void PatternTables::release()
+{
+    m_sizes.release();
+    m_tables.release();
 }
 
 void PatternTables::emit(cudaStream_t st)
@@ -115,7 +132,7 @@ void PatternTables::emit(cudaStream_t st)
     const size_t n = m_total.pieces;
     a.rec_stride = m_total.rec_words;
     const size_t win = n * 16 * sizeof(uint4), rec = n * a.rec_stride * 4;  // 16-byte multiples
-    m_tables.reserve(win + rec + n * sizeof(kern::PatternPiece));
+    m_tables.reserve(bytes());
     uint8_t* base = m_tables.get<uint8_t>();
     a.win = reinterpret_cast<uint4*>(base);
     a.rec = reinterpret_cast<uint32_t*>(base + win);
@@ -407,7 +424,14 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
         const size_t avail = free_b + m_tr.capacity() + m_q.capacity() + m_out[0].capacity() +
                              m_out[1].capacity() + m_stage[0].capacity() + m_stage[1].capacity();
         while (G > bt && bytes_for(G) > avail / 100 * 90) G = round_up(G / 2, bt);
-        if (bytes_for(G) > avail) DD_THROW(DEDISP_MEM_ALLOC_FAILED);
+        if (bytes_for(G) > avail) {
+            if (!s.pattern) DD_THROW(DEDISP_MEM_ALLOC_FAILED);
+            // the row-by-row form needs no tables, and half the rows at 16 bits
+            for (PatternTables& t : m_tables) t.release();
+            m_setup->pattern_ok = false;
+            execute(v, c);
+            return;
+        }
     }
 
     const size_t nbuf = nbuf_for(G);

@@ -71,13 +71,17 @@ public:
     enum Fit { kUse, kRowsFaster, kTooWide };
     // kTooWide: some group's rows do not fit the ring at this period (try a
     // shorter one); kRowsFaster: the row-by-row kernel needs fewer
-    // shared-memory wavefronts, or the tables exceed 2 GiB. Waits for `st`.
+    // shared-memory wavefronts, or the tables exceed 2 GiB or a quarter of the
+    // free device memory. Waits for `st`.
     Fit fit(cudaStream_t st);
+    // Bytes of the tables that emit() builds (after fit).
+    size_t bytes() const;
     // Row words of the widest group beyond its periods (after fit).
     long group_words() const { return (long)m_total.rows - (long)kern::kPatternGroup * 32 * m_args.lane_words; }
     void emit(cudaStream_t st);
     // Table arguments for the DM blocks from `block` on.
     void fill(kern::DedisperseArgs& a, size_t block) const;
+    void release();
 
 private:
     rt::DeviceBuffer m_sizes, m_tables;

@@ -67,3 +67,32 @@ def test_saturated_bytes_all_channels():
     delays = po.delay_table(nchans, np.float32(250e-6), np.float32(1500.0), np.float32(-0.02))
     ref = po.tdd(packed, nsamps, nchans, 8, nchans, delays, np.ones(nchans, np.int32), dms, 32, nout)
     assert np.array_equal(out.view(np.uint32), ref.view(np.uint32))
+
+
+def test_scarce_memory_takes_the_row_form():
+    """16-bit strided rows are twice the packed ones: with device memory for
+    1.4 times the packed rows only, a call gives what it gives with room."""
+    import torch
+    dt, f0, df = FINE
+    nchans, nout = 4096, 4096
+    dms = np.linspace(1480, 1500, 64).astype(np.float32)
+    p = dd.TDDPlan(nchans, dt, f0, df)
+    p.set_dm_list(dms)
+    nsamps = nout + p.get_max_delay()
+    x = torch.randint(0, 256, (nsamps, 2 * nchans), dtype=torch.uint8, device="cuda")
+    y = [torch.zeros((len(dms), nout), dtype=torch.float32, device="cuda") for _ in range(2)]
+    p.execute(nsamps, x, 16, y[0], 32, dd.DEDISP_DEVICE_POINTERS)
+    p.close()
+    p = dd.TDDPlan(nchans, dt, f0, df)
+    p.set_dm_list(dms)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    target = int(1.4 * (nchans + 1) * nsamps * 2)
+    free = torch.cuda.mem_get_info()[0]
+    block = torch.empty(free - target, dtype=torch.uint8, device="cuda")
+    try:
+        p.execute(nsamps, x, 16, y[1], 32, dd.DEDISP_DEVICE_POINTERS)
+    finally:
+        del block
+        torch.cuda.empty_cache()
+    assert torch.equal(y[0].view(torch.int32), y[1].view(torch.int32))
