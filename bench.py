@@ -997,14 +997,14 @@ def run_ours(args):
         raise RuntimeError("integer-pipe probe failed")
     k2_ms = sum(kms) / len(kms)
     adds = float(units) * cfg.nchans
-    # DRAM bytes per K2 launch: ncu captures (2026-12-03, --clock-control none)
-    # of each quad-strided shape on the same workload cut to 2^17 samples
+    # DRAM bytes per K2 launch: ncu captures (2026-12-03, variant 5 2026-12-05;
+    # --clock-control none) of each default or quad-strided shape on the same workload cut to 2^17 samples
     # (dram__bytes_read.sum + dram__bytes_write.sum of one launch), scaled by
     # the time tiles of the full launch (every tile streams its own delay
     # band, so the traffic grows with the tiles).
     # variant ({J, NW} of the library's quad shapes): (bytes in the capture,
     # time tiles in the capture, samples per tile = 128 J)
-    captured = {5: (10798106368 + 1397426944, 38, 2560),   # {20, 12}
+    captured = {5: (14403895000 + 1394524000, 47, 2048),   # shared group sums, period 512 words
                 6: (9808037376 + 1385468928, 34, 2816),    # {22, 12}
                 7: (11724679936 + 1397582848, 42, 2304),   # {18, 12}
                 8: (12990360064 + 1396900352, 47, 2048)}   # {16, 12}
@@ -1013,7 +1013,7 @@ def run_ours(args):
         b, tiles_cap, bt = captured[best]
         tiles = -(-nout // bt)
         traffic = round(b / tiles_cap * tiles)
-        traffic_note = (f"ncu capture 2026-12-03 of variant {best} on the workload cut to 2^17 samples "
+        traffic_note = (f"ncu capture of variant {best} on the workload cut to 2^17 samples "
                         f"({tiles_cap} tiles), scaled to this launch's {tiles} tiles; not measured "
                         f"in this run")
     achieved = adds / (k2_ms * 1e-3) / 1e12
@@ -1024,7 +1024,8 @@ def run_ours(args):
                 "peak_source": "measured in this run: dedisp_probe_alu (lib/libdedisp_probe.so; 32-bit add "
                                "lane-ops/s, all SMs)",
                 "k2_ms": round(k2_ms, 3), "k1_ms": round(sum(pms) / len(pms), 3),
-                "algorithmic": "nchan=4096 integer adds per DM-trial x sample; "
+                "algorithmic": "nchan=4096 integer adds per DM-trial x sample (variant 5 shares sums of "
+                               "channel groups between trials and so needs fewer: frac may pass 1); "
                                f"{adds:.3e} adds per step",
                 "hbm_view": {"algorithmic_bytes": int(cfg.nsamps * 4096 * args.nbits // 8 +
                                                       units * 4),
