@@ -1401,9 +1401,15 @@ __global__ void __launch_bounds__(MAC_THREADS) mac_plain_kernel(MacArgs a, int b
 // two bins neither gathers nor issue slots bind alone, the chain from delay to
 // sum does.
 //
+// One segment asks for two CTAs of 256 threads an SM, which fixes 128 registers
+// and lets the compiler keep more loads in flight than it chose by itself: 12.62
+// -> 12.41 ms at 512 DMs, 47.5 -> 45.1 at 2048. Wider tiles lose by it (four
+// segments 6.75 -> 7.03; 0 leaves them to the compiler, which at a bound of 1
+// would spend more registers: nine segments 14.4 -> 16.0).
+//
 // Measured on B200, 1024 channels, ms, tiled (one segment: 8 DMs a thread of 256)
 // -> here: 512 DMs x 16385 bins x 9 segments 74.6 -> 14.4; 2048 DMs x 39 segments
-// 336 -> 255; 512 DMs x 73728 bins x 1 segment 56.7 -> 12.6.
+// 336 -> 255; 512 DMs x 73728 bins x 1 segment 56.7 -> 12.4.
 constexpr int TAB_THREADS = 256;
 constexpr int TAB_CK = 128;      // channels staged at a time
 constexpr int TAB_MAX_TS = 10;
@@ -1417,7 +1423,7 @@ __device__ __forceinline__ float2 lds_float2(uint32_t addr)
 }
 
 template <int TS, int TM, bool MIRROR>
-__global__ void __launch_bounds__(TAB_THREADS) mac_table_kernel(MacArgs a, int dmax, int bins_per_block, int ts, int groups)
+__global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel(MacArgs a, int dmax, int bins_per_block, int ts, int groups)
 {
     extern __shared__ __align__(16) float2 s_tab[];
     const unsigned tab_n = ((unsigned)dmax + 2u) & ~1u;  // even counts keep the arrays aligned
