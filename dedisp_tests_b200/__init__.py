@@ -121,6 +121,7 @@ def lib() -> C.CDLL:
         "dedisp_b200_get_stage_times": (err, [_vp, C.POINTER(C.c_float), C.c_int]),
         "dedisp_b200_get_phasor_source": (err, [_vp, C.POINTER(C.c_int)]),
         "dedisp_b200_get_tc_form": (err, [_vp, C.POINTER(C.c_int)]),
+        "dedisp_b200_get_tdd_form": (err, [_vp] + 3 * [C.POINTER(C.c_int)]),
         "dedisp_b200_fdd_segment_length": (_sz, [_sz, _sz, _sz, _sz, C.c_int, _sz]),
         "dedisp_b200_set_wait_limit_ns": (err, [C.c_ulonglong]),
         "dedisp_b200_get_wait_limit_ns": (C.c_ulonglong, []),
@@ -295,6 +296,9 @@ class Plan:
         return self.TC_FORMS[v.value]
 
 
+TDD_FORMS = {-1: None, 0: "plain", 1: "rows", 2: "shared"}
+
+
 class DedispPlan(Plan):
     """Original dedisp interface (reference src/dedisp/DedispPlan.hpp)."""
     IMPLEMENTATION = DEDISP_DEDISP
@@ -306,6 +310,13 @@ class DedispPlan(Plan):
     def set_tile_variant(self, variant: int) -> None:
         """Tile shape of the tiled kernel for 8-bit input (same sums)."""
         _check(lib().dedisp_b200_set_tdd_variant(self._h, variant))
+
+    def get_form(self) -> tuple:
+        """Kernel of the last execute: (name, words per lane, most rounds of a
+        channel group); the counts are 0 unless the name is "shared"."""
+        v = [C.c_int() for _ in range(3)]
+        _check(lib().dedisp_b200_get_tdd_form(self._h, *[C.byref(x) for x in v]))
+        return (TDD_FORMS[v[0].value], v[1].value, v[2].value)
 
 
 class TDDPlan(DedispPlan):
@@ -393,6 +404,7 @@ _BATCH_SIGS = {
     "dedisp_b200_batch_set_timing": (C.c_int, [_vp, C.c_int]),
     "dedisp_b200_batch_get_timing": (C.c_int, [_vp, C.POINTER(C.c_float), C.POINTER(C.c_float),
                                                C.POINTER(C.c_int)]),
+    "dedisp_b200_batch_get_form": (C.c_int, [_vp] + 3 * [C.POINTER(C.c_int)]),
     "dedisp_b200_batch_max_delay": (_sz, [_vp, _sz]),
     "dedisp_b200_fdd_batch_create": (C.c_int, [C.POINTER(_vp), _sz, C.c_float, C.c_float, C.c_float,
                                                _sz, C.c_int]),
@@ -507,6 +519,12 @@ class Batch:
         _bcheck(_batch_lib().dedisp_b200_batch_get_timing(self._h, C.byref(a), C.byref(b),
                                                           C.byref(n)))
         return {"transpose_ms": a.value, "dedisperse_ms": b.value, "launches": n.value}
+
+    def get_form(self) -> tuple:
+        """Kernel of the last execute (see DedispPlan.get_form)."""
+        v = [C.c_int() for _ in range(3)]
+        _bcheck(_batch_lib().dedisp_b200_batch_get_form(self._h, *[C.byref(x) for x in v]))
+        return (TDD_FORMS[v[0].value], v[1].value, v[2].value)
 
     def max_delay(self, beam: int) -> int:
         return int(_batch_lib().dedisp_b200_batch_max_delay(self._h, beam))

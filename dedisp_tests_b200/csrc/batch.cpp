@@ -40,6 +40,7 @@ struct TddBatch::Layout {
     std::vector<size_t> pitch;                // words per channel row
     bool quad = false;                        // strided rows (quad variants, pattern kernel)
     bool pattern = false;                     // shared channel-group sums (tdd_pattern.hpp)
+    int rounds = 0;                           // pattern: most rounds of a channel group (upload)
     int period = 0;                           // quad: P words
     std::vector<size_t> q_off;                // quad: rows' offset in the workspace (words)
     std::vector<size_t> qpitch;               // quad: words per row
@@ -389,7 +390,10 @@ void TddBatch::upload(Layout& L)
         a.perm = t.perm.empty() ? nullptr : m_d_perm.get<int32_t>() + t.dm_off;
         a.out = t.spec.out;
         a.err = m_d_err.get<unsigned>();
-        if (L.pattern) m_tables[b]->fill(a, 0);
+        if (L.pattern) {
+            m_tables[b]->fill(a, 0);
+            L.rounds = std::max(L.rounds, m_tables[b]->rounds());
+        }
     }
     L.args = args;
     L.ws = ws;
@@ -449,6 +453,18 @@ void TddBatch::enqueue(cudaStream_t s, const Layout& L, bool timing)
     }
     if (timing) m_ev[2]->record(s);
     last_launches = launches;
+}
+
+TddStats TddBatch::form() const
+{
+    TddStats s;
+    if (!m_layout) return s;
+    s.form = m_layout->pattern ? 2 : m_layout->tiled ? 1 : 0;
+    if (m_layout->pattern) {
+        s.lane_words = m_layout->period / 32;
+        s.rounds = m_layout->rounds;
+    }
+    return s;
 }
 
 void TddBatch::sync(cudaStream_t stream)
@@ -708,6 +724,16 @@ dedisp_error dedisp_b200_batch_get_timing(dedisp_b200_batch batch, float* transp
         if (transpose_ms) *transpose_ms = b.last_k1_ms;
         if (dedisperse_ms) *dedisperse_ms = b.last_k2_ms;
         if (launches) *launches = b.last_launches;
+    });
+}
+
+dedisp_error dedisp_b200_batch_get_form(dedisp_b200_batch batch, int* form, int* lane_words, int* rounds)
+{
+    return batch_call(batch, [&](dedisp::detail::TddBatch& b) {
+        const dedisp::detail::TddStats s = b.form();
+        if (form) *form = s.form;
+        if (lane_words) *lane_words = s.lane_words;
+        if (rounds) *rounds = s.rounds;
     });
 }
 

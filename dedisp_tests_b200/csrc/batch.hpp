@@ -67,6 +67,9 @@ public:
     // wait of the last execute's dedispersion expired.
     void sync(cudaStream_t stream);
 
+    // Kernel of the last execute (codes and counts of TddStats).
+    TddStats form() const;
+
     size_t beam_count() const { return m_beams.size(); }
     size_t max_delay(size_t beam) const;
     size_t nsamp_out(size_t beam) const;

@@ -363,6 +363,18 @@ dedisp_error dedisp_b200_get_tc_form(dedisp_plan plan, int* form)
     return DEDISP_NO_ERROR;
 }
 
+dedisp_error dedisp_b200_get_tdd_form(dedisp_plan plan, int* form, int* lane_words, int* rounds)
+{
+    if (!plan) return DEDISP_INVALID_PLAN;
+    auto* g = dynamic_cast<dedisp::GPUPlan*>(plan->ptr.get());
+    if (!g) return DEDISP_INVALID_PLAN;
+    const dedisp::ExecTiming t = g->last_timing();
+    if (form) *form = t.tdd_form;
+    if (lane_words) *lane_words = t.lane_words;
+    if (rounds) *rounds = t.rounds;
+    return DEDISP_NO_ERROR;
+}
+
 dedisp_error dedisp_b200_last_error(char* msg, dedisp_size len)
 {
     if (msg && len) {

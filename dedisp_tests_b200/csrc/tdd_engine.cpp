@@ -357,6 +357,11 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     prepare(v, c);
     const Setup& s = *m_setup;
     stats.tiled = s.tiled;
+    stats.form = s.pattern ? 2 : s.tiled ? 1 : 0;
+    if (s.pattern) {
+        stats.lane_words = s.lane_words;
+        stats.rounds = m_tables[s.lane_words == 16 ? 0 : s.lane_words == 8 ? 1 : 2].rounds();
+    }
 
     const bool dev_in = (c.flags & DEDISP_DEVICE_POINTERS) != 0;
     const bool dev_out = dev_in;

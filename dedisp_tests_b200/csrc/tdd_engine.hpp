@@ -54,6 +54,9 @@ struct TddStats {
     float transpose_ms = 0.f;
     int launches = 0;
     bool tiled = false;
+    int form = -1;       // 0 plain, 1 row by row, 2 shared channel-group sums; -1 none ran
+    int lane_words = 0;  // form 2: words per lane
+    int rounds = 0;      // form 2: most rounds that a group took its trials in
 };
 
 // Whether the pattern kernel takes these (ascending) DMs and active channels'
@@ -74,6 +77,8 @@ public:
     // shared-memory wavefronts, or the tables exceed 2 GiB or a quarter of the
     // free device memory. Waits for `st`.
     Fit fit(cudaStream_t st);
+    // Most rounds that a group took its trials in (after fit).
+    int rounds() const { return (int)m_total.rounds; }
     // Bytes of the tables that emit() builds (after fit).
     size_t bytes() const;
     // Row words of the widest group beyond its periods (after fit).

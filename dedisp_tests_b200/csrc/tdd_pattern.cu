@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(128) pattern_size_kernel(PatternTableArgs a)
         atomicAdd(&a.totals->pieces, (unsigned)(D / p.sub));
         atomicMax(&a.totals->rec_words, (unsigned)rec);
         atomicMax(&a.totals->rows, (unsigned)p.rows);
+        atomicMax(&a.totals->rounds, (unsigned)(D / p.sub));
         atomicAdd(&a.block[blk].y, (unsigned)(D / p.sub));
     }
 }

@@ -21,7 +21,8 @@ struct PatternTotals {
     unsigned rec_words;       // longest record
     unsigned next;            // pieces handed out
     unsigned rows;            // row words of the widest group
-    unsigned pad[2];          // (the block counts follow, 16-byte aligned)
+    unsigned rounds;          // most rounds of a group
+    unsigned pad;             // (the block counts follow, 16-byte aligned)
 };
 
 // One piece of a DM block's walk: a channel group, or a round of its trials.

@@ -74,6 +74,9 @@ ExecTiming TDDPlan::last_timing() const
     t.prep_ms = m_engine->stats.transpose_ms;
     t.launches = m_engine->stats.launches;
     t.variant = m_engine->stats.tiled ? 1 : 0;
+    t.tdd_form = m_engine->stats.form;
+    t.lane_words = m_engine->stats.lane_words;
+    t.rounds = m_engine->stats.rounds;
     return t;
 }
 
@@ -148,6 +151,9 @@ ExecTiming DedispPlan::last_timing() const
     t.prep_ms = m_engine->stats.transpose_ms;
     t.launches = m_engine->stats.launches;
     t.variant = m_engine->stats.tiled ? 1 : 0;
+    t.tdd_form = m_engine->stats.form;
+    t.lane_words = m_engine->stats.lane_words;
+    t.rounds = m_engine->stats.rounds;
     return t;
 }
 

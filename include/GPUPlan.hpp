@@ -35,6 +35,12 @@ struct ExecTiming {
      * K step, 1 fused, 2 three MMAs with 3 A buffers, 3 CTA pairs (M = 256),
      * 4 CTA pairs with 3 A buffers, 5 fused at 64-channel chunks); -1 none */
     int tc_form = -1;
+    /* TDD plans: kernel of the last execute (0 plain, 1 row by row, 2 shared
+     * channel-group sums; -1 none), and of form 2 the words per lane and the
+     * most rounds that a channel group took its trials in */
+    int tdd_form = -1;
+    int lane_words = 0;
+    int rounds = 0;
 };
 
 class GPUPlan : public Plan {

@@ -38,6 +38,12 @@ dedisp_error dedisp_b200_set_tdd_kernel(dedisp_plan plan, int kernel);
 dedisp_error dedisp_b200_set_tdd_variant(dedisp_plan plan, int variant);
 int dedisp_b200_tdd_variant_count(dedisp_size in_nbits);
 
+/* DEDISP_DEDISP / DEDISP_TDD plans: kernel of the last execute: 0 plain, 1 row
+ * by row (the tiled variants), 2 shared channel-group sums; -1 none ran. Of
+ * form 2 also its words per lane (4, 8 or 16) and the most rounds (1, 2, 4 or
+ * 8) in which a channel group took its trials, else 0. Pointers may be NULL. */
+dedisp_error dedisp_b200_get_tdd_form(dedisp_plan plan, int* form, int* lane_words, int* rounds);
+
 /* Runs the plan's device work on a caller-provided cudaStream_t (NULL
  * restores the plan's own stream). */
 dedisp_error dedisp_b200_set_stream(dedisp_plan plan, void* cuda_stream);
@@ -204,6 +210,8 @@ dedisp_error dedisp_b200_batch_sync(dedisp_b200_batch batch, void* stream);
 dedisp_error dedisp_b200_batch_set_timing(dedisp_b200_batch batch, int enable);
 dedisp_error dedisp_b200_batch_get_timing(dedisp_b200_batch batch, float* transpose_ms,
                                           float* dedisperse_ms, int* launches);
+/* Kernel of the last execute, as dedisp_b200_get_tdd_form. */
+dedisp_error dedisp_b200_batch_get_form(dedisp_b200_batch batch, int* form, int* lane_words, int* rounds);
 dedisp_size dedisp_b200_batch_max_delay(dedisp_b200_batch batch, dedisp_size beam);
 /* The batch functions return their specific error code; the message of the
  * last failure on the calling thread is available from dedisp_b200_last_error. */
