@@ -437,7 +437,10 @@ __device__ __forceinline__ void pattern_stage(const DedisperseArgs& a, size_t t0
         if (p + 2 < pieces && lane <= G) next[1] = __ldg(win + (size_t)(p + 2) * 16 + lane);
         const int after = (int)__shfl_sync(FULL, c.y, 0);
         const uint32_t slot = __shfl_sync(FULL, c.w, 0);
-        if (after >= 0 && !piece_wait(y.summed, after, wc.ns)) {
+        // (the warp leaves as one: a lane that went on alone would wait for the
+        // others in the next shuffle for good)
+        const bool ok = after < 0 || piece_wait(y.summed, after, wc.ns);
+        if (!__all_sync(FULL, ok)) {
             if (lane == 0) atomicExch(&y.failed, 1);
             return;
         }
