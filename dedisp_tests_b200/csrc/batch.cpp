@@ -242,7 +242,7 @@ void TddBatch::set_shape(const BatchShape& shape)
 size_t TddBatch::max_delay(size_t beam) const { return m_beams.at(beam).max_delay; }
 size_t TddBatch::nsamp_out(size_t beam) const { return m_beams.at(beam).nout; }
 
-TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limit) const
+TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limit, bool shared) const
 {
     Layout L;
     L.shape = shape;
@@ -251,7 +251,7 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
     const bool want_tiled = !m_general_mask;
     // the default shape, sized by the library, is the pattern kernel where
     // that is the faster one
-    L.pattern = want_tiled && m_pattern && v == kern::tiled_default_variant(nb) && shape.chan_per_stage == 0;
+    L.pattern = shared && want_tiled && m_pattern && v == kern::tiled_default_variant(nb) && shape.chan_per_stage == 0;
     const size_t bd = L.pattern ? (size_t)kern::kPatternDms : (size_t)kern::tiled_block_dms(nb, v);
     const size_t bt = L.pattern ? (size_t)kern::pattern_block_samples(nb, m_lane_words) : (size_t)kern::tiled_block_samples(nb, v);
     const int J = kern::tiled_lane_words(nb, v);
@@ -347,20 +347,33 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
     return L;
 }
 
-size_t TddBatch::workspace_bytes() const
+TddBatch::Layout TddBatch::fitting_layout(const BatchShape& shape, size_t tile_limit) const
 {
-    size_t words = 0;
+    Layout L = make_layout(shape, tile_limit);
+    if (!m_ext_ws) return L;  // its own grows to workspace_bytes()
+    if (L.pattern && L.ws_words > m_ext_ws_bytes / 4) L = make_layout(shape, tile_limit, false);
+    if (L.ws_words > m_ext_ws_bytes / 4)
+        DD_THROW_MSG(DEDISP_MEM_ALLOC_FAILED, "workspace too small for the current beams");
+    return L;
+}
+
+size_t TddBatch::workspace_words(bool shared) const
+{
+    size_t words = 64;
     for (int v = 0; v < kern::tiled_batch_variant_count(m_nbits); ++v) {
         BatchShape s;
         s.variant = v;
-        words = std::max(words, make_layout(s, 0).ws_words);
+        words = std::max(words, make_layout(s, 0, shared).ws_words);
     }
-    return std::max<size_t>(words, 64) * 4;
+    return words;
 }
+
+size_t TddBatch::workspace_bytes() const { return workspace_words(true) * 4; }
 
 void TddBatch::set_workspace(void* ptr, size_t bytes)
 {
-    if (ptr && bytes < workspace_bytes()) DD_THROW_MSG(DEDISP_MEM_ALLOC_FAILED, "workspace too small");
+    if (ptr && bytes / 4 < workspace_words(false))
+        DD_THROW_MSG(DEDISP_MEM_ALLOC_FAILED, "workspace too small");
     m_ext_ws = ptr;
     m_ext_ws_bytes = ptr ? bytes : 0;
     m_dirty = true;
@@ -494,7 +507,7 @@ BatchShape TddBatch::autotune(cudaStream_t stream)
     BatchShape best_shape = m_shape;
     std::vector<int> fit_cs;  // stage sizes of the current variant's largest-fit layout
     for (const BatchShape& c : cands) {
-        Layout L = make_layout(c, kTuneSamples);
+        Layout L = fitting_layout(c, kTuneSamples);
         std::vector<int> cs;
         for (auto& a : L.args) cs.push_back(a.chan_per_stage);
         if (c.chan_per_stage == 0) fit_cs = cs;
@@ -526,7 +539,7 @@ void TddBatch::execute(cudaStream_t stream, bool use_graph)
     if (m_beams.empty()) return;
     if (m_dirty || !m_layout) {
         drop_graph();
-        m_layout.reset(new Layout(make_layout(m_shape, 0)));
+        m_layout.reset(new Layout(fitting_layout(m_shape, 0)));
         upload(*m_layout);
         m_dirty = false;
     }

@@ -54,7 +54,9 @@ public:
 
     // Device bytes of transposed-input scratch needed by any tile shape.
     size_t workspace_bytes() const;
-    // Caller-owned scratch (device, >= workspace_bytes()); nullptr: own.
+    // Caller-owned scratch (device); nullptr: own. It has to hold every
+    // row-by-row shape of the current beams; shared channel-group sums run in it
+    // where their rows fit too (workspace_bytes()). Every execute checks it.
     void set_workspace(void* ptr, size_t bytes);
 
     // Times every candidate shape on the leading time tiles of all beams
@@ -85,7 +87,12 @@ public:
 private:
     struct BeamState;
     struct Layout;
-    Layout make_layout(const BatchShape& shape, size_t tile_limit_samples) const;
+    // The layout of a shape; `shared` false keeps the row-by-row form.
+    Layout make_layout(const BatchShape& shape, size_t tile_limit_samples, bool shared = true) const;
+    // The same within the caller's workspace: row by row where the shared sums'
+    // rows do not fit it, DEDISP_MEM_ALLOC_FAILED where neither does.
+    Layout fitting_layout(const BatchShape& shape, size_t tile_limit_samples) const;
+    size_t workspace_words(bool shared) const;
     void upload(Layout& L);
     void prepare_patterns();
     void enqueue(cudaStream_t s, const Layout& L, bool timing);

@@ -183,7 +183,10 @@ dedisp_error dedisp_b200_batch_set_beams(dedisp_b200_batch batch, const dedisp_b
                                          dedisp_size nbeams);
 /* Scratch for the transposed inputs (any tile shape); a caller may hand the
  * same buffer to several batches that it runs one after another on one
- * stream. Without one the batch allocates its own. */
+ * stream. Without one the batch allocates its own. The size follows the beams,
+ * the killmask and the kernel that they get; every execute checks it: a batch
+ * whose shared-sum rows do not fit runs row by row, and one that has no form
+ * that fits fails with DEDISP_MEM_ALLOC_FAILED. */
 dedisp_size dedisp_b200_batch_workspace_size(dedisp_b200_batch batch);
 dedisp_error dedisp_b200_batch_set_workspace(dedisp_b200_batch batch, void* d_workspace,
                                              dedisp_size bytes);
