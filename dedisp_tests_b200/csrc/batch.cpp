@@ -363,7 +363,9 @@ size_t TddBatch::workspace_words(bool shared) const
     for (int v = 0; v < kern::tiled_batch_variant_count(m_nbits); ++v) {
         BatchShape s;
         s.variant = v;
-        words = std::max(words, make_layout(s, 0, shared).ws_words);
+        words = std::max(words, make_layout(s, 0, false).ws_words);
+        // the default variant has a second layout with the shared sums
+        if (shared) words = std::max(words, make_layout(s, 0).ws_words);
     }
     return words;
 }

@@ -194,7 +194,7 @@ dedisp_error dedisp_b200_batch_set_workspace(dedisp_b200_batch batch, void* d_wo
  * per stage even and <= 32 (0: the largest that fits shared memory; the
  * quad-strided variants size their stages per block and ignore it). The default
  * variant with 0 runs the kernel on shared channel-group sums where that is the
- * faster one for every beam. */
+ * faster one for every beam; with any other count it runs row by row. */
 int dedisp_b200_batch_variant_count(dedisp_size in_nbits);
 dedisp_error dedisp_b200_batch_set_shape(dedisp_b200_batch batch, int variant, int chan_per_stage);
 /* Times every candidate shape on the leading 8192 output samples of each

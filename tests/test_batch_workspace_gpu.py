@@ -77,3 +77,25 @@ def test_longer_beams_are_refused():
     b.set_workspace(None, 0)
     check(b, ins2, outs2, [dms], 8)
     assert ws.intact()
+
+
+@pytest.mark.parametrize("nbits,nout,shapes", [
+    (8, 2816, [(5, 16), (5, 0)]),   # just past a 2560-sample tile: longer rows than the shared sums'
+    (2, 2700, [(1, 8), (1, 0)]),
+    (16, 200, [(0, 24), (0, 16), (0, 0)]),  # packed rows of 448-sample blocks
+])
+def test_workspace_holds_every_shape(nbits, nout, shapes):
+    """The default variant has two layouts, shared sums (0 channels per stage)
+    and row by row (any other count): the workspace holds both."""
+    lists = [fine_list(64, step=0.4)] if nbits == 8 else [fine_list(40)]
+    b, ins, outs, _ = make_batch(nbits, lists, [nout])
+    ws = Workspace(b.workspace_size())
+    b.set_workspace(ws.buf, ws.n)
+    for shape in shapes:
+        b.set_shape(*shape)
+        check(b, ins, outs, lists, nbits)
+        assert b.get_form()[0] == ("rows" if shape[1] else "shared"), shape
+        assert ws.intact(), shape
+    b.autotune()
+    check(b, ins, outs, lists, nbits)
+    assert ws.intact()
