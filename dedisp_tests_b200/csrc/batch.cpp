@@ -180,25 +180,41 @@ void TddBatch::set_beams(std::vector<BatchBeamSpec> beams)
 }
 
 // Pattern tables of every beam; the default shape uses the pattern kernel if
-// it takes each of them and is the faster one for each.
+// it takes each of them and is the faster one for each. Otherwise, and where
+// they cannot be had, no tables are kept and the batch runs row by row.
 void TddBatch::prepare_patterns()
 {
     m_pattern = false;
-    if (m_general_mask || m_beams.empty() || m_chan.empty()) return;
+    bool built = false;
+    try {
+        built = build_patterns();
+    } catch (const Error& e) {
+        m_pattern = false;
+        m_tables.clear();
+        if (e.code() != DEDISP_MEM_ALLOC_FAILED) throw;
+        cudaGetLastError();  // taken care of: nothing was lost but the tables
+    }
+    if (!built) m_tables.clear();
+    m_pattern = built;
+}
+
+bool TddBatch::build_patterns()
+{
+    if (m_general_mask || m_beams.empty() || m_chan.empty()) return false;
     std::vector<float> cdl(m_chan.size());
     for (size_t j = 0; j < cdl.size(); ++j) cdl[j] = m_delays[m_chan[j]];
     long words = 0;
     size_t tiles = 0;
     const size_t bt = (size_t)kern::pattern_block_samples(m_nbits, 4);
     for (const BeamState& t : m_beams) {
-        if (!pattern_takes(t.sorted, cdl, m_nbits)) return;
+        if (!pattern_takes(t.sorted, cdl, m_nbits)) return false;
         tiles += (t.sorted.size() + kern::kPatternDms - 1) / kern::kPatternDms * ((t.nout + bt - 1) / bt);
     }
     // a period at which every beam's groups fit
     bool wide = true;
     while (wide) {
         m_lane_words = kern::pattern_lane_words(m_nbits, tiles, words);
-        if (!m_lane_words) return;
+        if (!m_lane_words) return false;
         m_tables.resize(m_beams.size());
         for (size_t b = 0; b < m_beams.size(); ++b) {
             const BeamState& t = m_beams[b];
@@ -210,23 +226,26 @@ void TddBatch::prepare_patterns()
         for (auto& t : m_tables) {
             const PatternTables::Fit fit = t->fit(nullptr);
             words = std::max(words, t->group_words());
-            if (fit == PatternTables::kRowsFaster) return;
+            if (fit == PatternTables::kRowsFaster) return false;
             if (fit == PatternTables::kTooWide) wide = true;
         }
     }
-    // room for all tables and the workspace, else the row-by-row form
-    size_t tables = 0, free_b = 0, total_b = 0;
-    for (auto& t : m_tables) tables += t->bytes();
-    RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
-    m_pattern = true;
-    const size_t ws = m_ext_ws ? 0 : workspace_bytes(), held = m_own_ws.capacity();
-    if (tables > free_b / 4 || (ws > held && ws + tables > free_b + held)) {
-        m_pattern = false;
-        m_tables.clear();
-        return;
+    // room for all tables (beside those held from earlier beams) and the
+    // workspace, else the row-by-row form
+    size_t tables = 0, tables_held = 0, free_b = 0, total_b = 0;
+    for (auto& t : m_tables) {
+        tables += t->bytes();
+        tables_held += t->held();
     }
+    RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
+    m_pattern = true;  // workspace_bytes() counts their rows
+    const size_t ws = m_ext_ws ? 0 : workspace_bytes(), held = m_own_ws.capacity();
+    m_pattern = false;
+    free_b += tables_held;
+    if (tables > free_b / 4 || (ws > held && ws + tables > free_b + held)) return false;
     for (auto& t : m_tables) t->emit(nullptr);
     RT_CHECK(cudaStreamSynchronize(nullptr));
+    return true;
 }
 
 void TddBatch::set_shape(const BatchShape& shape)

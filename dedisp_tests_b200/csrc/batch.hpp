@@ -95,6 +95,7 @@ private:
     size_t workspace_words(bool shared) const;
     void upload(Layout& L);
     void prepare_patterns();
+    bool build_patterns();
     void enqueue(cudaStream_t s, const Layout& L, bool timing);
     void drop_graph();
     uint8_t* workspace_base();

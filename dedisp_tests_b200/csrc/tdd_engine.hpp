@@ -81,6 +81,8 @@ public:
     int rounds() const { return (int)m_total.rounds; }
     // Bytes of the tables that emit() builds (after fit).
     size_t bytes() const;
+    // Bytes held for them now.
+    size_t held() const { return m_tables.capacity(); }
     // Row words of the widest group beyond its periods (after fit).
     long group_words() const { return (long)m_total.rows - (long)kern::kPatternGroup * 32 * m_args.lane_words; }
     void emit(cudaStream_t st);
