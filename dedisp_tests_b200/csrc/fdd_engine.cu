@@ -36,6 +36,7 @@ struct FddEngine::Impl {
     int dmax = -1;               // largest delay index, -1 if any DM is negative or NaN
     int nact = 0;
     std::vector<float> delays_active;
+    bool delays_ok = false;      // none of them negative or NaN (a band that runs past zero frequency)
 };
 
 FddEngine::FddEngine(GpuState& gpu) : m_gpu(gpu), m_impl(new Impl()) {}
@@ -99,6 +100,7 @@ void FddEngine::execute(const FddOptions& opt, const FddView& v, const FddCall& 
         RT_CHECK(cudaMemcpy(m.delay_act.get(), dl.data(), n * 4, cudaMemcpyHostToDevice));
         RT_CHECK(cudaMemcpy(m.dms.get(), v.dms, ndm * 4, cudaMemcpyHostToDevice));
         m.delays_active.assign(dl.begin(), dl.begin() + m.nact);
+        m.delays_ok = std::all_of(m.delays_active.begin(), m.delays_active.end(), [](float d) { return d >= 0.f; });
         m.version = v.version;
     }
     const bool use_tc = opt.precision == FddPrecision::BF16x3 && m.nact > 0;
@@ -324,9 +326,10 @@ void FddEngine::execute(const FddOptions& opt, const FddView& v, const FddCall& 
         a.nfft = (unsigned)g.nfft;
         a.round_delays = opt.round_delays ? 1 : 0;
         a.tw = tw;
-        // the per-bin phasor table where it fits (DMs without negative delays,
-        // max delays up to about 20000), else phasors from the twiddle tables
-        if (kern::fdd_mac_table_fits(m.dmax, (unsigned)g.nfft, (int)ndm, m.nact, (int)nseg))
+        // the per-bin phasor table where it fits (DMs and delays that are not
+        // negative, max delays up to about 20000), else phasors from the
+        // twiddle tables
+        if (m.delays_ok && kern::fdd_mac_table_fits(m.dmax, (unsigned)g.nfft, (int)ndm, m.nact, (int)nseg))
             kern::launch_fdd_mac_table(a, m.dmax, st);
         else
             kern::launch_fdd_mac_plain(a, st);

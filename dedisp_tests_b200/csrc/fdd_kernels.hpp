@@ -123,8 +123,10 @@ struct MacArgs {
 };
 void launch_fdd_mac_plain(const MacArgs& a, cudaStream_t s);
 // The same sums with a per-bin phasor table over delays 0..dmax (the largest
-// delay index of the plan's DMs and channels). fdd_mac_table_fits: dmax known,
-// the tables fit, and building them is not the larger part of the work.
+// delay index of the plan's DMs and channels). No DM and no delay may be
+// negative or NaN: the kernel reads the table without a check of the index.
+// fdd_mac_table_fits: dmax known, the tables fit, and building them is not the
+// larger part of the work.
 bool fdd_mac_table_fits(int dmax, unsigned nfft, int ndm, int nact, int nseg);
 void launch_fdd_mac_table(const MacArgs& a, int dmax, cudaStream_t s);
 
