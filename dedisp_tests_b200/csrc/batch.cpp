@@ -219,8 +219,9 @@ bool TddBatch::build_patterns()
         for (size_t b = 0; b < m_beams.size(); ++b) {
             const BeamState& t = m_beams[b];
             if (!m_tables[b]) m_tables[b].reset(new PatternTables());
-            m_tables[b]->size(m_d_dms.get<float>() + t.dm_off, t.sorted.size(), m_d_chan.get<int32_t>(),
-                              m_d_cdl.get<float>(), m_chan.size(), m_nchans, m_nbits, m_lane_words, nullptr);
+            if (!m_tables[b]->size(m_d_dms.get<float>() + t.dm_off, t.sorted.size(), m_d_chan.get<int32_t>(),
+                                   m_d_cdl.get<float>(), m_chan.size(), m_nchans, m_nbits, m_lane_words, nullptr))
+                return false;
         }
         wide = false;
         for (auto& t : m_tables) {
@@ -243,7 +244,8 @@ bool TddBatch::build_patterns()
     m_pattern = false;
     free_b += tables_held;
     if (tables > free_b / 4 || (ws > held && ws + tables > free_b + held)) return false;
-    for (auto& t : m_tables) t->emit(nullptr);
+    for (auto& t : m_tables)
+        if (!t->emit(nullptr)) return false;
     RT_CHECK(cudaStreamSynchronize(nullptr));
     return true;
 }

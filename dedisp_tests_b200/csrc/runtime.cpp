@@ -76,6 +76,24 @@ void DeviceBuffer::reserve(size_t bytes)
     m_cap = bytes;
 }
 
+bool DeviceBuffer::reserve_optional(size_t bytes)
+{
+    if (bytes <= m_cap) return true;
+    size_t free_b = 0, total_b = 0;
+    RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
+    if (bytes > (free_b + m_cap) / 4) return false;
+    release();
+    const cudaError_t e = cudaMalloc(&m_ptr, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();  // taken care of by the caller
+        m_ptr = nullptr;
+        return false;
+    }
+    RT_CHECK(e);
+    m_cap = bytes;
+    return true;
+}
+
 void DeviceBuffer::release()
 {
     if (m_ptr) cudaFree(m_ptr);

@@ -47,6 +47,10 @@ public:
 
     // Ensures capacity >= bytes; contents are not preserved on growth.
     void reserve(size_t bytes);
+    // reserve() for what the caller can do without: growth takes at most a
+    // quarter of the memory that is free (with what the buffer holds); false,
+    // with the buffer unchanged or empty, where that is not enough.
+    bool reserve_optional(size_t bytes);
     void release();
     template <typename T = void>
     T* get() const { return static_cast<T*>(m_ptr); }

@@ -16,6 +16,7 @@ namespace {
 constexpr int kMaxOutGroups = 8;                   // DM groups for D2H overlap
 
 size_t round_up(size_t a, size_t b) { return (a + b - 1) / b * b; }
+int table_index(int lane_words) { return lane_words == 16 ? 0 : lane_words == 8 ? 1 : 2; }
 }  // namespace
 
 bool pattern_takes(const std::vector<float>& dms, const std::vector<float>& delays, int nbits)
@@ -63,14 +64,14 @@ struct TddEngine::Setup {
     std::vector<int32_t> perm;   // output row of each slot
 };
 
-void PatternTables::size(const float* d_dms, size_t ndm, const int32_t* d_chan, const float* d_delay, size_t nact,
+bool PatternTables::size(const float* d_dms, size_t ndm, const int32_t* d_chan, const float* d_delay, size_t nact,
                          size_t zero_row, int nbits, int lane_words, cudaStream_t st)
 {
     const size_t nblk = (ndm + kern::kPatternDms - 1) / kern::kPatternDms;
     const size_t ngroups = (nact + kern::kPatternGroup - 1) / kern::kPatternGroup;
     const size_t head = sizeof(kern::PatternTotals) + nblk * sizeof(uint4);
     static_assert(sizeof(kern::PatternTotals) % sizeof(uint4) == 0, "block counts follow the totals");
-    m_sizes.reserve(head + nblk * ngroups * sizeof(int4));
+    if (!m_sizes.reserve_optional(head + nblk * ngroups * sizeof(int4))) return false;
     m_nbits = nbits;
     kern::PatternTableArgs a{};
     a.dms = d_dms;
@@ -93,6 +94,7 @@ void PatternTables::size(const float* d_dms, size_t ndm, const int32_t* d_chan, 
     a.size = reinterpret_cast<int4*>(base + head);
     kern::launch_pattern_sizes(a, st);
     m_args = a;
+    return true;
 }
 
 PatternTables::Fit PatternTables::fit(cudaStream_t st)
@@ -105,14 +107,7 @@ PatternTables::Fit PatternTables::fit(cudaStream_t st)
     // samples apart, 2 bits: 0.240 ms here against 0.231 at nearly equal
     // wavefronts; 5% below them the two are even).
     const unsigned long long rows = (unsigned long long)m_args.ndm * m_args.nact * m_args.lane_words;
-    if (m_total.cost * 8 >= rows * 7 || bytes() > ((size_t)2 << 30)) return kRowsFaster;
-    if (bytes() > m_tables.capacity()) {
-        // where memory is scarce it is left to the rows and outputs
-        size_t free_b = 0, total_b = 0;
-        RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
-        if (bytes() > (free_b + m_tables.capacity()) / 4) return kRowsFaster;
-    }
-    return kUse;
+    return m_total.cost * 8 >= rows * 7 || bytes() > ((size_t)2 << 30) ? kRowsFaster : kUse;
 }
 
 size_t PatternTables::bytes() const
@@ -126,18 +121,19 @@ void PatternTables::release()
     m_tables.release();
 }
 
-void PatternTables::emit(cudaStream_t st)
+bool PatternTables::emit(cudaStream_t st)
 {
     kern::PatternTableArgs& a = m_args;
     const size_t n = m_total.pieces;
     a.rec_stride = m_total.rec_words;
     const size_t win = n * 16 * sizeof(uint4), rec = n * a.rec_stride * 4;  // 16-byte multiples
-    m_tables.reserve(bytes());
+    if (!m_tables.reserve_optional(bytes())) return false;
     uint8_t* base = m_tables.get<uint8_t>();
     a.win = reinterpret_cast<uint4*>(base);
     a.rec = reinterpret_cast<uint32_t*>(base + win);
     a.sched = reinterpret_cast<kern::PatternPiece*>(base + win + rec);
     kern::launch_pattern_tables(a, m_total.pieces, st);
+    return true;
 }
 
 void PatternTables::fill(kern::DedisperseArgs& a, size_t block) const
@@ -275,25 +271,42 @@ void TddEngine::choose_form(const TddView& v, const TddCall& c)
         cudaStream_t st = m_gpu.stream();
         int J = kern::pattern_lane_words(c.in_nbits, tiles, s.group_words), i = 0;
         for (; J; J = kern::pattern_lane_words(c.in_nbits, tiles, s.group_words)) {
-            i = J == 16 ? 0 : J == 8 ? 1 : 2;
+            i = table_index(J);
             if (s.table[i]) break;
             PatternTables& t = m_tables[i];
-            t.size(m_dms.get<float>(), s.dms.size(), m_chan.get<int32_t>(), m_cdl.get<float>(), (size_t)s.nact,
-                   v.nchans, c.in_nbits, J, st);
-            const PatternTables::Fit fit = t.fit(st);
-            s.group_words = t.group_words();
-            if (fit == PatternTables::kTooWide) continue;  // a shorter period, if one fits
-            s.table[i] = fit == PatternTables::kUse ? 1 : -1;
-            if (fit == PatternTables::kUse) t.emit(st);
+            bool use = t.size(m_dms.get<float>(), s.dms.size(), m_chan.get<int32_t>(), m_cdl.get<float>(),
+                              (size_t)s.nact, v.nchans, c.in_nbits, J, st);
+            if (use) {
+                const PatternTables::Fit fit = t.fit(st);
+                s.group_words = t.group_words();
+                if (fit == PatternTables::kTooWide) continue;  // a shorter period, if one fits
+                use = fit == PatternTables::kUse && t.emit(st);
+            }
+            s.table[i] = use ? 1 : -1;
             break;
         }
         s.pattern = J && s.table[i] == 1;
         s.lane_words = J;
     }
+    // a list or mask that takes the row-by-row form keeps no tables
+    if (!s.pattern && s.table[0] != 1 && s.table[1] != 1 && s.table[2] != 1) drop_idle_tables();
     if (!s.pattern) size_rows(v, c.in_nbits);
     s.tiled = s.pattern || s.rows_tiled;
     s.quad = s.pattern || s.rows_quad;
     s.period = s.pattern ? 32 * s.lane_words : s.rows_period;
+}
+
+bool TddEngine::drop_idle_tables()
+{
+    Setup& s = *m_setup;
+    bool any = false;
+    for (int i = 0; i < 3; ++i) {
+        if (s.pattern && i == table_index(s.lane_words)) continue;
+        any = any || m_tables[i].held() > 0;
+        m_tables[i].release();
+        s.table[i] = std::min(s.table[i], 0);
+    }
+    return any;
 }
 
 // Window and stage sizes of the row-by-row tiled form, and its padded channel
@@ -360,7 +373,7 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     stats.form = s.pattern ? 2 : s.tiled ? 1 : 0;
     if (s.pattern) {
         stats.lane_words = s.lane_words;
-        stats.rounds = m_tables[s.lane_words == 16 ? 0 : s.lane_words == 8 ? 1 : 2].rounds();
+        stats.rounds = m_tables[table_index(s.lane_words)].rounds();
     }
 
     const bool dev_in = (c.flags & DEDISP_DEVICE_POINTERS) != 0;
@@ -426,8 +439,12 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     if (!held) {
         size_t free_b = 0, total_b = 0;
         RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
-        const size_t avail = free_b + m_tr.capacity() + m_q.capacity() + m_out[0].capacity() +
-                             m_out[1].capacity() + m_stage[0].capacity() + m_stage[1].capacity();
+        const size_t own = m_tr.capacity() + m_q.capacity() + m_out[0].capacity() + m_out[1].capacity() +
+                           m_stage[0].capacity() + m_stage[1].capacity();
+        // tables of other calls go before the gulp shrinks
+        if (bytes_for(G) > (free_b + own) / 100 * 90 && drop_idle_tables())
+            RT_CHECK(cudaMemGetInfo(&free_b, &total_b));
+        const size_t avail = free_b + own;
         while (G > bt && bytes_for(G) > avail / 100 * 90) G = round_up(G / 2, bt);
         if (bytes_for(G) > avail) {
             if (!s.pattern) DD_THROW(DEDISP_MEM_ALLOC_FAILED);
@@ -577,7 +594,7 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
                 da.out = out_base;
             }
             if (s.pattern) {
-                m_tables[s.lane_words == 16 ? 0 : s.lane_words == 8 ? 1 : 2].fill(da, s0 / bd);  // s0 is a multiple of bd
+                m_tables[table_index(s.lane_words)].fill(da, s0 / bd);  // s0 is a multiple of bd
                 kern::launch_dedisperse_pattern(da, ex);
             } else if (s.tiled) kern::launch_dedisperse_tiled(da, ex);
             else kern::launch_dedisperse_plain(da, ex);

@@ -69,13 +69,13 @@ bool pattern_takes(const std::vector<float>& dms, const std::vector<float>& dela
 // enqueues the tables.
 class PatternTables {
 public:
-    void size(const float* d_dms, size_t ndm, const int32_t* d_chan, const float* d_delay, size_t nact,
+    // (false: no memory for its sizes)
+    bool size(const float* d_dms, size_t ndm, const int32_t* d_chan, const float* d_delay, size_t nact,
               size_t zero_row, int nbits, int lane_words, cudaStream_t st);
     enum Fit { kUse, kRowsFaster, kTooWide };
     // kTooWide: some group's rows do not fit the ring at this period (try a
     // shorter one); kRowsFaster: the row-by-row kernel needs fewer
-    // shared-memory wavefronts, or the tables exceed 2 GiB or a quarter of the
-    // free device memory. Waits for `st`.
+    // shared-memory wavefronts, or the tables exceed 2 GiB. Waits for `st`.
     Fit fit(cudaStream_t st);
     // Most rounds that a group took its trials in (after fit).
     int rounds() const { return (int)m_total.rounds; }
@@ -85,7 +85,9 @@ public:
     size_t held() const { return m_tables.capacity(); }
     // Row words of the widest group beyond its periods (after fit).
     long group_words() const { return (long)m_total.rows - (long)kern::kPatternGroup * 32 * m_args.lane_words; }
-    void emit(cudaStream_t st);
+    // (false: no memory for the tables, or more than a quarter of what is free:
+    // it is left to the rows and outputs)
+    bool emit(cudaStream_t st);
     // Table arguments for the DM blocks from `block` on.
     void fill(kern::DedisperseArgs& a, size_t block) const;
     void release();
@@ -122,6 +124,9 @@ private:
     void prepare(const TddView& v, const TddCall& c);
     void choose_form(const TddView& v, const TddCall& c);
     void size_rows(const TddView& v, int nbits);
+    // Gives back the tables that the current form does not use; true if there
+    // were any.
+    bool drop_idle_tables();
 
     GpuState& m_gpu;
     std::unique_ptr<Setup> m_setup;

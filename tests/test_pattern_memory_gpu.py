@@ -72,3 +72,30 @@ def test_batch_counts_held_tables_as_room():
     finally:
         del block
         torch.cuda.empty_cache()
+
+
+def test_plan_gives_tables_back():
+    fine, coarse = beams(FINE, COARSE)
+    p = dd.TDDPlan(*PARAMS)
+
+    def run(beam, tries=1):
+        p.set_dm_list(beam[3])
+        for _ in range(tries):
+            p.execute(beam[2], beam[0], 8, beam[4], 32, dd.DEDISP_DEVICE_POINTERS)
+            if p.get_form()[0] == "shared":
+                break
+        return p.get_form()[0]
+
+    p.set_tile_variant(6)             # a row-by-row variant: the buffers, no tables
+    assert run(fine) == "rows"
+    before = free_bytes()
+    p.set_tile_variant(5)             # the default one
+    assert run(fine, 64) == "shared"
+    held = before - free_bytes()
+    assert held > 8 << 20
+    assert run(coarse) == "rows"      # this list takes no tables
+    assert before - free_bytes() < held // 2
+    assert run(fine, 64) == "shared"
+    p.set_tile_variant(6)             # nor does this variant
+    assert run(fine) == "rows"
+    assert before - free_bytes() < held // 2
