@@ -108,17 +108,42 @@ size_t StreamServer::start()
     RT_CHECK(cudaDeviceSynchronize());
     size_t free0 = 0, total = 0;
     RT_CHECK(cudaMemGetInfo(&free0, &total));
-    size_t ndm_max = 0, md_max = 0;
+    size_t ndm_max = 0;
     for (auto& b : m_beams) {
         ndm_max = std::max(ndm_max, b->dms.size());
-        md_max = std::max(md_max, b->max_delay);
         for (auto& r : b->ring) {
             r.reserve((b->max_delay + m_cfg.max_gulp) * m_row_bytes);
             RT_CHECK(cudaMemset(r.get(), 0, (b->max_delay + m_cfg.max_gulp) * m_row_bytes));
         }
     }
-    // Workers: one plan per DM-list group of the worker's kind, sized by a
-    // warm-up at the largest gulp on zero rows.
+    // Above the budget once more without the shared-sum tables of TDD plans,
+    // which run row by row then.
+    for (const bool tables : {true, false}) {
+        m_workers.clear();
+        make_workers(tables, ndm_max);
+        RT_CHECK(cudaDeviceSynchronize());
+        size_t free1 = 0;
+        RT_CHECK(cudaMemGetInfo(&free1, &total));
+        m_bytes = free0 > free1 ? free0 - free1 : 0;
+        if (!m_cfg.hbm_budget || m_bytes <= m_cfg.hbm_budget || m_cfg.tdd_workers == 0) break;
+    }
+    if (m_cfg.hbm_budget && m_bytes > m_cfg.hbm_budget)
+        DD_THROW_MSG(DEDISP_MEM_ALLOC_FAILED, ("server needs " + std::to_string(m_bytes) +
+                                               " device bytes, above the budget").c_str());
+    m_started = true;
+    for (auto& w : m_workers) {
+        Worker* wp = w.get();
+        w->thread = std::thread([this, wp] { worker_loop(wp); });
+    }
+    return m_bytes;
+}
+
+// Workers: one plan per DM-list group of the worker's kind, sized by a warm-up
+// at the largest gulp on zero rows. The warm-up also decides the kernel of every
+// later gulp: a shorter one would take tables of another period, and the first
+// such gulp would allocate and wait for them.
+void StreamServer::make_workers(bool tables, size_t ndm_max)
+{
     const int nw = m_cfg.tdd_workers + m_cfg.fdd_workers;
     for (int i = 0; i < nw; ++i) {
         std::unique_ptr<Worker> w(new Worker);
@@ -133,6 +158,7 @@ size_t StreamServer::start()
             std::unique_ptr<Plan> p;
             if (w->kind == 0) {
                 auto* t = new TDDPlan(m_cfg.nchans, m_cfg.dt, m_cfg.f0, m_cfg.df, m_cfg.device);
+                t->set_tables(tables ? TDDPlan::Tables::FirstCall : TDDPlan::Tables::None);
                 p.reset(t);
             } else {
                 auto* f = new FDDGPUPlan(m_cfg.nchans, m_cfg.dt, m_cfg.f0, m_cfg.df, m_cfg.device);
@@ -154,19 +180,6 @@ size_t StreamServer::start()
         }
         m_workers.push_back(std::move(w));
     }
-    RT_CHECK(cudaDeviceSynchronize());
-    size_t free1 = 0;
-    RT_CHECK(cudaMemGetInfo(&free1, &total));
-    m_bytes = free0 > free1 ? free0 - free1 : 0;
-    if (m_cfg.hbm_budget && m_bytes > m_cfg.hbm_budget)
-        DD_THROW_MSG(DEDISP_MEM_ALLOC_FAILED, ("server needs " + std::to_string(m_bytes) +
-                                               " device bytes, above the budget").c_str());
-    m_started = true;
-    for (auto& w : m_workers) {
-        Worker* wp = w.get();
-        w->thread = std::thread([this, wp] { worker_loop(wp); });
-    }
-    return m_bytes;
 }
 
 long StreamServer::submit(int beam, const uint8_t* rows, size_t n, float* d_out)

@@ -92,6 +92,7 @@ private:
         float* d_out;
         double t_submit;
     };
+    void make_workers(bool tables, size_t ndm_max);
     void worker_loop(Worker* w);
     void run_job(Worker* w, const Job& j, GulpRecord& rec);
 

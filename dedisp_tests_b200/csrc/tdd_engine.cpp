@@ -47,6 +47,7 @@ struct TddEngine::Setup {
     int rows_period = 0;
 
     // form of the current call
+    bool form_chosen = false;
     bool tiled = false;
     bool quad = false;           // strided rows (quad kernels, pattern kernel)
     bool pattern = false;        // shared channel-group sums (tdd_pattern.hpp)
@@ -259,12 +260,13 @@ void TddEngine::prepare(const TddView& v, const TddCall& c)
 void TddEngine::choose_form(const TddView& v, const TddCall& c)
 {
     Setup& s = *m_setup;
+    if (keep_form && s.form_chosen) return;
     s.pattern = false;
     // an explicitly tiled plan is refused where the row-by-row form is
     if (kernel == TddKernel::Tiled) size_rows(v, c.in_nbits);
     if (kernel == TddKernel::Tiled && !s.rows_tiled)
         DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "tiled kernel unavailable for this killmask/DM list");
-    if (s.pattern_ok) {
+    if (s.pattern_ok && use_tables) {
         const size_t nout = std::min(c.nsamps - v.max_delay, gulp_set && gulp_size ? gulp_size : kDefaultGulp);
         const size_t bt = (size_t)kern::pattern_block_samples(c.in_nbits, 4);
         const size_t tiles = (s.dms.size() + kern::kPatternDms - 1) / kern::kPatternDms * ((nout + bt - 1) / bt);
@@ -294,6 +296,7 @@ void TddEngine::choose_form(const TddView& v, const TddCall& c)
     s.tiled = s.pattern || s.rows_tiled;
     s.quad = s.pattern || s.rows_quad;
     s.period = s.pattern ? 32 * s.lane_words : s.rows_period;
+    s.form_chosen = true;
 }
 
 bool TddEngine::drop_idle_tables()

@@ -117,6 +117,8 @@ public:
     TddKernel kernel = TddKernel::Auto;
     int variant = -1;  // tile-shape variant of the tiled kernel (8-bit input; -1: default)
     bool record_timing = false;
+    bool use_tables = true;   // the pattern kernel may run
+    bool keep_form = false;   // the first call of a setup decides the form of all
     TddStats stats;
 
 private:

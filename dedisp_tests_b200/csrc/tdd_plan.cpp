@@ -66,6 +66,11 @@ void TDDPlan::set_gulp_size(size_type gulp_size)
 dedisp_size TDDPlan::get_gulp_size() const { return m_engine->gulp_size; }
 void TDDPlan::set_kernel(TddKernel k) { m_engine->kernel = k; }
 void TDDPlan::set_tile_variant(int variant) { m_engine->variant = variant; }
+void TDDPlan::set_tables(Tables t)
+{
+    m_engine->use_tables = t != Tables::None;
+    m_engine->keep_form = t == Tables::FirstCall;
+}
 void TDDPlan::set_timing(bool enable) { m_engine->record_timing = enable; }
 ExecTiming TDDPlan::last_timing() const
 {

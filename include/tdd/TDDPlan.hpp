@@ -56,6 +56,12 @@ public:
                             dedisp_size dm_count, unsigned flags);
     void set_kernel(TddKernel k);
     void set_tile_variant(int variant);
+    /* The tables of the shared channel-group sums (extension): as each call
+     * pays for them, or decided by the first call on a DM list and kept for
+     * every later one of at most its length, which then allocates nothing; or
+     * none. */
+    enum class Tables { PerCall, FirstCall, None };
+    void set_tables(Tables t);
     void set_timing(bool enable) override;
     ExecTiming last_timing() const override;
 
