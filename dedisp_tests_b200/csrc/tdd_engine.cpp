@@ -475,7 +475,6 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     uint32_t* tr = m_tr.get<uint32_t>();
     if (quad) {
         m_err.reserve(sizeof(unsigned));
-        m_err_host.reserve(sizeof(unsigned));
         RT_CHECK(cudaMemsetAsync(m_err.get(), 0, sizeof(unsigned), ex));
     }
 
@@ -625,12 +624,14 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
 
     const bool async = (c.flags & DEDISP_ASYNC) && dev_in;
     if (!async) {
-        // the error word comes back behind the kernels, before the one wait
-        if (quad)
-            RT_CHECK(cudaMemcpyAsync(m_err_host.get(), m_err.get(), sizeof(unsigned), cudaMemcpyDeviceToHost, ex));
+        // the error word comes back behind the kernels, before the one wait (to
+        // pageable memory, which that copy waits for by itself: a pinned word
+        // per plan cost 2 to 9 ms at the plan's first call)
+        unsigned failed = 0;
+        if (quad) RT_CHECK(cudaMemcpyAsync(&failed, m_err.get(), sizeof(failed), cudaMemcpyDeviceToHost, ex));
         RT_CHECK(cudaStreamSynchronize(ex));
         if (!dev_out) RT_CHECK(cudaStreamSynchronize(d2h));
-        if (quad && *m_err_host.get<unsigned>())
+        if (failed)
             DD_THROW_MSG(DEDISP_INTERNAL_GPU_ERROR, "a staged window copy did not complete");
     }
     if (record_timing) {
