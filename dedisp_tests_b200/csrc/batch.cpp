@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <limits>
+#include <map>
 #include <numeric>
 
 #include "dedisp_b200.h"
@@ -29,7 +30,27 @@ struct TddBatch::BeamState {
     size_t nout = 0;
     uint32_t tmax = 0;           // largest delay over active channels and DMs
     size_t dm_off = 0;           // offset in the concatenated device DM / perm arrays
+    mutable std::map<size_t, uint32_t> spans;  // delay_span of each block size asked for
 };
+
+// Largest difference of a channel's delays over a block of `bd` DMs. Kept per
+// block size: it takes two delays per channel and block on the host, and a
+// workspace size asks for every variant's layout.
+uint32_t TddBatch::delay_span(const BeamState& t, size_t bd) const
+{
+    const auto known = t.spans.find(bd);
+    if (known != t.spans.end()) return known->second;
+    uint32_t span = 0;
+    for (size_t i = 0; i < t.sorted.size(); i += bd) {
+        const float f = t.sorted[i], l = t.sorted[std::min(i + bd, t.sorted.size()) - 1];
+        for (int32_t c : m_chan) {
+            const uint32_t x = hostmath::delay_rn(f, m_delays[c]), y = hostmath::delay_rn(l, m_delays[c]);
+            span = std::max(span, x > y ? x - y : y - x);
+        }
+    }
+    t.spans[bd] = span;
+    return span;
+}
 
 struct TddBatch::Layout {
     BatchShape shape;
@@ -98,6 +119,7 @@ void TddBatch::set_killmask(const int32_t* killmask)
     if (killmask) std::copy(killmask, killmask + m_nchans, m_km.begin());
     m_chan.clear();
     m_kmv.clear();
+    for (BeamState& b : m_beams) b.spans.clear();
     m_general_mask = false;
     for (size_t c = 0; c < m_nchans; ++c) {
         if (m_km[c] == 0) continue;
@@ -293,14 +315,7 @@ TddBatch::Layout TddBatch::make_layout(const BatchShape& shape, size_t tile_limi
     bool tiled = want_tiled;
     for (size_t b = 0; b < nbeams && tiled && !L.pattern; ++b) {
         const BeamState& t = m_beams[b];
-        uint32_t span = 0;
-        for (size_t i = 0; i < t.sorted.size(); i += bd) {
-            const float f = t.sorted[i], l = t.sorted[std::min(i + bd, t.sorted.size()) - 1];
-            for (int32_t c : m_chan) {
-                const uint32_t x = hostmath::delay_rn(f, m_delays[c]), y = hostmath::delay_rn(l, m_delays[c]);
-                span = std::max(span, x > y ? x - y : y - x);
-            }
-        }
+        const uint32_t span = delay_span(t, bd);
         // quad-strided rows: a 1-sample delay is a 1-word offset
         const size_t w = quad ? round_up((size_t)span + 3 + 32 * (size_t)J, 4)
                               : round_up((span + 4 * (size_t)spw - 1) / spw + 32 * (size_t)J + 1, 4);

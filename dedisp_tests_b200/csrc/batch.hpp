@@ -93,6 +93,7 @@ private:
     // rows do not fit it, DEDISP_MEM_ALLOC_FAILED where neither does.
     Layout fitting_layout(const BatchShape& shape, size_t tile_limit_samples) const;
     size_t workspace_words(bool shared) const;
+    uint32_t delay_span(const BeamState& t, size_t block_dms) const;
     void upload(Layout& L);
     void prepare_patterns();
     bool build_patterns();
