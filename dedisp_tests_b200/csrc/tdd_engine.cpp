@@ -14,6 +14,15 @@ namespace detail {
 
 namespace {
 constexpr int kMaxOutGroups = 8;                   // DM groups for D2H overlap
+// A DM range, mask or width that is new to the plan costs the shared sums 0.1 to
+// 0.3 ms of tables, and where they decline 0.1 ms to know it. From about 2e9
+// additions (trials x channels x samples, 0.2 ms row by row) one call earns that
+// back; a smaller one runs row by row and leaves the tables to the next call on
+// the same setup. Calls alternating over two ranges, ms, tables at once against
+// none: 64 channels x 32 trials x 8192 samples 0.117 and 0.092, 256 x 32 x 16384
+// (declined) 0.25 and 0.136, 1024 x 32 x 62914 0.355 and 0.385, 1024 x 512 x
+// 62914 1.06 and 1.72.
+constexpr double kTablesAtOnce = 2e9;
 
 size_t round_up(size_t a, size_t b) { return (a + b - 1) / b * b; }
 int table_index(int lane_words) { return lane_words == 16 ? 0 : lane_words == 8 ? 1 : 2; }
@@ -48,6 +57,7 @@ struct TddEngine::Setup {
 
     // form of the current call
     bool form_chosen = false;
+    bool tables_due = false;     // row by row for now, the tables at a later call
     bool tiled = false;
     bool quad = false;           // strided rows (quad kernels, pattern kernel)
     bool pattern = false;        // shared channel-group sums (tdd_pattern.hpp)
@@ -235,9 +245,10 @@ void TddEngine::prepare(const TddView& v, const TddCall& c)
                    pattern_takes(n.dms, cdl, c.in_nbits);
     m_dms.reserve(n.dms.size() * 4);
     RT_CHECK(cudaMemcpyAsync(m_dms.get(), n.dms.data(), n.dms.size() * 4, cudaMemcpyHostToDevice, st));
-    m_chan.reserve(chan.size() * 4);
+    // (room for the padding that size_rows adds)
+    m_chan.reserve((chan.size() + 256) * 4);
     RT_CHECK(cudaMemcpyAsync(m_chan.get(), chan.data(), chan.size() * 4, cudaMemcpyHostToDevice, st));
-    m_cdl.reserve(cdl.size() * 4);
+    m_cdl.reserve((cdl.size() + 256) * 4);
     RT_CHECK(cudaMemcpyAsync(m_cdl.get(), cdl.data(), cdl.size() * 4, cudaMemcpyHostToDevice, st));
     std::vector<uint32_t> km(n.km_vals);
     if (km.empty()) km.push_back(0);
@@ -262,6 +273,8 @@ void TddEngine::choose_form(const TddView& v, const TddCall& c)
     Setup& s = *m_setup;
     if (keep_form && s.form_chosen) return;
     s.pattern = false;
+    const bool first_call = !s.form_chosen;
+    s.tables_due = false;
     // an explicitly tiled plan is refused where the row-by-row form is
     if (kernel == TddKernel::Tiled) size_rows(v, c.in_nbits);
     if (kernel == TddKernel::Tiled && !s.rows_tiled)
@@ -271,10 +284,19 @@ void TddEngine::choose_form(const TddView& v, const TddCall& c)
         const size_t bt = (size_t)kern::pattern_block_samples(c.in_nbits, 4);
         const size_t tiles = (s.dms.size() + kern::kPatternDms - 1) / kern::kPatternDms * ((nout + bt - 1) / bt);
         cudaStream_t st = m_gpu.stream();
+        auto later = [&] {
+            if (first_call && !keep_form && (double)s.dms.size() * s.nact * (double)nout < kTablesAtOnce) return true;
+            // tables take an allocation and a wait, which a capture must not see
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            RT_CHECK(cudaStreamIsCapturing(st, &cap));
+            return cap != cudaStreamCaptureStatusNone;
+        };
         int J = kern::pattern_lane_words(c.in_nbits, tiles, s.group_words), i = 0;
         for (; J; J = kern::pattern_lane_words(c.in_nbits, tiles, s.group_words)) {
             i = table_index(J);
             if (s.table[i]) break;
+            s.tables_due = later();
+            if (s.tables_due) break;
             PatternTables& t = m_tables[i];
             bool use = t.size(m_dms.get<float>(), s.dms.size(), m_chan.get<int32_t>(), m_cdl.get<float>(),
                               (size_t)s.nact, v.nchans, c.in_nbits, J, st);
@@ -291,7 +313,7 @@ void TddEngine::choose_form(const TddView& v, const TddCall& c)
         s.lane_words = J;
     }
     // a list or mask that takes the row-by-row form keeps no tables
-    if (!s.pattern && s.table[0] != 1 && s.table[1] != 1 && s.table[2] != 1) drop_idle_tables();
+    if (!s.pattern && !s.tables_due && s.table[0] != 1 && s.table[1] != 1 && s.table[2] != 1) drop_idle_tables();
     if (!s.pattern) size_rows(v, c.in_nbits);
     s.tiled = s.pattern || s.rows_tiled;
     s.quad = s.pattern || s.rows_quad;
@@ -463,7 +485,18 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     const size_t pitch = pitch_for(G);
     if (!quad) m_tr.reserve((v.nchans + 1) * pitch * 4);
     const size_t qpitch = quad ? qpitch_for(G) : 0;
-    if (quad) m_q.reserve((v.nchans + 1) * qpitch * 4);
+    if (quad) {
+        // room for the shared sums' rows too where they are still to come: a
+        // captured graph of this call keeps its buffer when they do
+        size_t words = 0;
+        if (s.tables_due)
+            for (int J : {4, 8, 16}) {
+                const size_t b = (size_t)kern::pattern_block_samples(nbits, J);
+                words = std::max(words, round_up(round_up(G, b) + s.tmax + 32 * (size_t)J + 32, 32));
+            }
+        if (words <= qpitch || !m_q.reserve_optional((v.nchans + 1) * words * 4))
+            m_q.reserve((v.nchans + 1) * qpitch * 4);
+    }
     for (size_t b = 0; b < nbuf; ++b) {
         if (!dev_out) m_out[b].reserve(ndm * G * ob);
         if (!dev_in) m_stage[b].reserve(in_bytes_for(G));
