@@ -56,6 +56,7 @@ struct TddEngine::Setup {
     int rows_period = 0;
 
     // form of the current call
+    size_t gulp = 0;             // output samples per pass
     bool form_chosen = false;
     bool tables_due = false;     // row by row for now, the tables at a later call
     bool tiled = false;
@@ -155,6 +156,98 @@ void PatternTables::fill(kern::DedisperseArgs& a, size_t block) const
     a.block = m_args.block + block;
     a.lane_words = m_args.lane_words;
 }
+
+// Host-buffer calls: time of a pass over the output samples, from the copies and
+// the tiles of a form.
+struct TddHostCall {
+    size_t nout, ndm, tmax;      // output samples, trials, largest delay
+    size_t row_bytes, out_bytes; // of an input row, of an output sample of all trials
+    size_t nchans;
+    bool identity;               // output rows in the order of the trials
+    size_t block_samples, block_dms;
+    double tile_us;              // one tile
+    size_t sms;
+    double copy_rate;            // bytes per us, either way
+};
+
+namespace {
+// Rates of a B200 on its host's bus: pinned buffers 52 GB/s either way, 72 both
+// ways together, pageable ones 10; the kernels' rows are made at 3 TB/s.
+constexpr double kPinnedBytesPerUs = 52e3, kPageableBytesPerUs = 10e3, kBothBytesPerUs = 72e3, kRowBytesPerUs = 3e6;
+// One tile, us a channel (1024 and 4096 channels): row by row 0.18, packed rows of
+// 16 bits 0.32 and of 32 bits 0.24; the plain kernel's small tiles 0.04 (at 2e12
+// additions a second); shared sums 0.093 at 4 words per lane, 0.100 at 8, 0.183
+// at 16.
+double rows_tile_us(int nact, int nbits) { return nact * (nbits == 16 ? 0.32 : nbits == 32 ? 0.24 : 0.18); }
+double plain_tile_us(int nact) { return 0.04 * nact; }
+double pattern_tile_us(int nact, int lane_words) { return nact * (0.06 + 0.0075 * lane_words); }
+
+double waves(size_t tiles, size_t sms) { return (double)((tiles + sms - 1) / sms); }
+
+// DM groups of the last gulp, so that its device-to-host copy starts group by
+// group. A group's launch takes whole waves of tiles; what shows is the first
+// group and all copies, or all groups and the last copy.
+size_t last_gulp_groups(const TddHostCall& h, size_t gc)
+{
+    const size_t blocks = (h.ndm + h.block_dms - 1) / h.block_dms;
+    const size_t across = (gc + h.block_samples - 1) / h.block_samples;
+    const double copy_us = (double)gc * (double)h.out_bytes / h.copy_rate;
+    size_t best = 1;
+    double least = 0;
+    for (size_t n = 1; n <= std::min<size_t>(h.identity ? kMaxOutGroups : 1, blocks); ++n) {
+        const double group = waves((blocks + n - 1) / n * across, h.sms) * h.tile_us + 10.0;
+        const double us = std::max(group + copy_us, (double)n * group + copy_us / (double)n);
+        if (n == 1 || us < least) {
+            best = n;
+            least = us;
+        }
+    }
+    return best;
+}
+
+// The gulps (first output sample, samples) of a call in gulps of G. With host
+// input and several gulps the first is a quarter of G: its input copy is the one
+// that no kernel hides, and the next gulp's copy runs during its kernels.
+std::vector<std::pair<size_t, size_t>> gulp_list(size_t nout, size_t G, size_t bt, bool host_in)
+{
+    std::vector<std::pair<size_t, size_t>> gulps;
+    for (size_t g0 = 0; g0 < nout;) {
+        size_t gc = std::min(G, nout - g0);
+        if (g0 == 0 && host_in && gc < nout && G >= 4 * bt) gc = round_up(G / 4, bt);
+        gulps.emplace_back(g0, gc);
+        g0 += gc;
+    }
+    return gulps;
+}
+
+// Two input and two output buffers, one stream each for the copies in, the
+// kernels and the copies out.
+double host_call_us(const TddHostCall& h, size_t G)
+{
+    double in[2] = {0, 0}, kern[2] = {0, 0}, out[2] = {0, 0};  // ends of the last two gulps
+    double in_bytes = 0;
+    const auto gulps = gulp_list(h.nout, G, h.block_samples, true);
+    const size_t blocks = (h.ndm + h.block_dms - 1) / h.block_dms;
+    for (size_t i = 0; i < gulps.size(); ++i) {
+        const size_t gc = gulps[i].second, a = i & 1;  // a: two gulps ago, then this one
+        const double bytes = (double)(gc + h.tmax) * (double)h.row_bytes;
+        in_bytes += bytes;
+        in[a] = std::max(in[a ^ 1], kern[a]) + bytes / h.copy_rate + 8.0;
+        double k = std::max({in[a], kern[a ^ 1], out[a]}) + (double)(gc + h.tmax) * (double)(4 * h.nchans + h.row_bytes) / kRowBytesPerUs;
+        double o = out[a ^ 1];
+        const size_t n = i + 1 == gulps.size() ? last_gulp_groups(h, gc) : 1;
+        const size_t across = (gc + h.block_samples - 1) / h.block_samples;
+        for (size_t g = 0; g < n; ++g) {
+            k += waves((blocks + n - 1) / n * across, h.sms) * h.tile_us + 10.0;
+            o = std::max(o, k) + (double)gc * (double)h.out_bytes / h.copy_rate / (double)n;
+        }
+        kern[a] = k;
+        out[a] = o;
+    }
+    const double both = (in_bytes + (double)h.nout * (double)h.out_bytes) / kBothBytesPerUs;
+    return std::max({out[0], out[1], both});
+}
+}  // namespace
 
 TddEngine::TddEngine(GpuState& gpu) : m_gpu(gpu), m_setup(new Setup()) {}
 TddEngine::~TddEngine()
@@ -271,7 +364,10 @@ void TddEngine::prepare(const TddView& v, const TddCall& c)
 void TddEngine::choose_form(const TddView& v, const TddCall& c)
 {
     Setup& s = *m_setup;
-    if (keep_form && s.form_chosen) return;
+    if (keep_form && s.form_chosen) {
+        choose_gulp(v, c, s.pattern);
+        return;
+    }
     s.pattern = false;
     const bool first_call = !s.form_chosen;
     s.tables_due = false;
@@ -280,12 +376,15 @@ void TddEngine::choose_form(const TddView& v, const TddCall& c)
     if (kernel == TddKernel::Tiled && !s.rows_tiled)
         DD_THROW_MSG(DEDISP_UNKNOWN_ERROR, "tiled kernel unavailable for this killmask/DM list");
     if (s.pattern_ok && use_tables) {
-        const size_t nout = std::min(c.nsamps - v.max_delay, gulp_set && gulp_size ? gulp_size : kDefaultGulp);
+        choose_gulp(v, c, true);
+        const size_t nout = s.gulp;
         const size_t bt = (size_t)kern::pattern_block_samples(c.in_nbits, 4);
         const size_t tiles = (s.dms.size() + kern::kPatternDms - 1) / kern::kPatternDms * ((nout + bt - 1) / bt);
         cudaStream_t st = m_gpu.stream();
         auto later = [&] {
-            if (first_call && !keep_form && (double)s.dms.size() * s.nact * (double)nout < kTablesAtOnce) return true;
+            if (first_call && !keep_form &&
+                (double)s.dms.size() * s.nact * (double)(c.nsamps - v.max_delay) < kTablesAtOnce)
+                return true;
             // tables take an allocation and a wait, which a capture must not see
             cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
             RT_CHECK(cudaStreamIsCapturing(st, &cap));
@@ -319,6 +418,72 @@ void TddEngine::choose_form(const TddView& v, const TddCall& c)
     s.quad = s.pattern || s.rows_quad;
     s.period = s.pattern ? 32 * s.lane_words : s.rows_period;
     s.form_chosen = true;
+    if (!s.pattern) choose_gulp(v, c, false);
+}
+
+// Output samples per pass: the user's cap, else the default, and for pinned host
+// buffers, whose copies overlap the kernels, the gulps that take the least time
+// in the model above (of the shared sums, or of the other forms) where that is at
+// least 2% less than one gulp's. Pageable copies wait in the driver: no gain.
+// Measured, ms, in one gulp; in eight or fewer of at least four times the overlap,
+// whatever the trials and tiles; here: 1024 channels x 512 trials x 50000 samples
+// 3.31, 4.03, 2.47; 1024 x 8 x 50000 (the input copy binds) 1.33, 1.92, 1.34;
+// 4096 x 200 x 100000 12.4, 14.4, 10.5; 4096 x 16 x 20000 (each gulp a wave of
+// 0.7 ms tiles) 3.0, 3.5, 2.4.
+void TddEngine::choose_gulp(const TddView& v, const TddCall& c, bool shared)
+{
+    Setup& s = *m_setup;
+    const bool host = !(c.flags & DEDISP_DEVICE_POINTERS), set = gulp_set && gulp_size;
+    const size_t nout = c.nsamps - v.max_delay;
+    s.gulp = std::min(nout, set ? gulp_size : host ? kHostDefaultGulp : kDefaultGulp);
+    if (!host || set || !m_pinned) return;
+    double least = 0.98 * host_call_us(host_call(v, c, shared, s.gulp), s.gulp);
+    const size_t one = s.gulp;
+    for (size_t k : {2, 3, 4, 6, 8, 12}) {
+        size_t G = (nout + k - 1) / k;
+        if (G >= one) continue;
+        const TddHostCall h = host_call(v, c, shared, G);
+        if (G > h.block_samples) G = G / h.block_samples * h.block_samples;
+        const double us = host_call_us(h, G);
+        if (us < least) {
+            least = us;
+            s.gulp = G;
+        }
+    }
+}
+
+// The model's numbers for a call in gulps of `gulp`, with the period that they
+// would get.
+TddHostCall TddEngine::host_call(const TddView& v, const TddCall& c, bool shared, size_t gulp) const
+{
+    const Setup& s = *m_setup;
+    TddHostCall h{};
+    h.nout = c.nsamps - v.max_delay;
+    h.ndm = s.dms.size();
+    h.tmax = s.tmax;
+    h.row_bytes = v.nchans * (size_t)c.in_nbits / 8;
+    h.out_bytes = h.ndm * (size_t)c.out_nbits / 8;
+    h.nchans = v.nchans;
+    h.identity = s.identity;
+    h.sms = (size_t)kern::tdd_sm_count();
+    h.copy_rate = m_pinned ? kPinnedBytesPerUs : kPageableBytesPerUs;
+    if (shared) {
+        h.block_dms = kern::kPatternDms;
+        const size_t b = (size_t)kern::pattern_block_samples(c.in_nbits, 4);
+        const size_t tiles = (h.ndm + h.block_dms - 1) / h.block_dms * ((gulp + b - 1) / b);
+        const int J = std::max(4, kern::pattern_lane_words(c.in_nbits, tiles, s.group_words));
+        h.block_samples = (size_t)kern::pattern_block_samples(c.in_nbits, J);
+        h.tile_us = pattern_tile_us(s.nact, J);
+    } else if (s.rows_tiled) {
+        h.block_samples = (size_t)kern::tiled_block_samples(c.in_nbits, s.variant);
+        h.block_dms = (size_t)kern::tiled_block_dms(c.in_nbits, s.variant);
+        h.tile_us = rows_tile_us(s.nact, c.in_nbits);
+    } else {
+        h.block_samples = 16;
+        h.block_dms = 32;
+        h.tile_us = plain_tile_us(s.nact);
+    }
+    return h;
 }
 
 bool TddEngine::drop_idle_tables()
@@ -392,6 +557,7 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
 
     const size_t nsamp_out = c.nsamps - v.max_delay;
     if (nsamp_out == 0 || c.dm_count == 0) return;
+    m_pinned = !(c.flags & DEDISP_DEVICE_POINTERS) && rt::is_pinned_host(c.in) && rt::is_pinned_host(c.out);
     prepare(v, c);
     const Setup& s = *m_setup;
     stats.tiled = s.tiled;
@@ -416,22 +582,11 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
                                 : 16;
     const size_t win = s.tiled && !s.pattern ? (size_t)s.win_words : 0;
 
-    // Gulp size: the user cap, the grid limit, then device memory. With more
-    // than one gulp the input rows and the output rows of a gulp have two
+    // Gulp size: as chosen with the form, the grid limit, then device memory. With
+    // more than one gulp the input rows and the output rows of a gulp have two
     // buffers each, so that gulp g+1's host-to-device copy and gulp g-1's
     // device-to-host copy run while gulp g is dedispersed.
-    size_t gulp_default = dev_in && dev_out ? kDefaultGulp : kHostDefaultGulp;
-    if (!dev_in && !(gulp_set && gulp_size)) {
-        // Pinned buffers: at least eight gulps, so that the input copies, the
-        // kernels and the output copies of a call of up to 2^18 samples overlap
-        // as well (1024 channels, 512 trials, 259522 samples: 16.4 ms in one
-        // gulp, 12.4 in nine), but each at least four times the overlap rows
-        // that it copies again. Pageable copies wait in the driver: no gain.
-        const size_t fine = std::max<size_t>({nsamp_out / 8, 4 * (size_t)s.tmax, 8192});
-        if (fine < std::min(nsamp_out, gulp_default) && rt::is_pinned_host(c.in) && rt::is_pinned_host(c.out))
-            gulp_default = fine;
-    }
-    size_t G = std::min(nsamp_out, gulp_set && gulp_size ? gulp_size : gulp_default);
+    size_t G = s.gulp;
     G = std::min(G, (size_t)65535 * bt);
     if (G < nsamp_out && G > bt) G = G / bt * bt;  // whole time tiles in every gulp but the last
     auto pitch_for = [&](size_t g) {
@@ -518,21 +673,14 @@ void TddEngine::execute(const TddView& v, const TddCall& c)
     // The last gulp's K2 runs per group of DM slots whose output rows are
     // contiguous, so that its device-to-host copy starts group by group
     // (every other gulp's copy already overlaps the next gulp's kernels, and
-    // each extra launch ends with a partly filled wave).
+    // each extra launch ends with a partly filled wave: last_gulp_groups).
     const size_t bd = s.tiled && !s.pattern ? (size_t)kern::tiled_block_dms(nbits, s.variant) : 32;
     const size_t ntile = (ndm + bd - 1) / bd;
-    const size_t ngroups_last = (!dev_out && s.identity) ? std::min<size_t>(kMaxOutGroups, ntile) : 1;
+    size_t ngroups_last = (!dev_out && s.identity) ? std::min<size_t>(kMaxOutGroups, ntile) : 1;
 
-    // Gulps (first output sample, samples). With host input and several
-    // gulps the first is a quarter of G: its input copy is the one that no
-    // kernel hides, and the next gulp's copy runs during its kernels.
-    std::vector<std::pair<size_t, size_t>> gulps;
-    for (size_t g0 = 0; g0 < nsamp_out;) {
-        size_t gc = std::min(G, nsamp_out - g0);
-        if (g0 == 0 && !dev_in && gc < nsamp_out && G >= 4 * bt) gc = round_up(G / 4, bt);
-        gulps.emplace_back(g0, gc);
-        g0 += gc;
-    }
+    const std::vector<std::pair<size_t, size_t>> gulps = gulp_list(nsamp_out, G, bt, !dev_in);
+    if (ngroups_last > 1)
+        ngroups_last = last_gulp_groups(host_call(v, c, s.pattern, G), gulps.back().second);
 
     std::unique_ptr<rt::Event> t_a, t_b, t_c;
     if (record_timing) {

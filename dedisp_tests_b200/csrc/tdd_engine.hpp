@@ -59,6 +59,8 @@ struct TddStats {
     int rounds = 0;      // form 2: most rounds that a group took its trials in
 };
 
+struct TddHostCall;  // model of a host-buffer call (tdd_engine.cpp)
+
 // Whether the pattern kernel takes these (ascending) DMs and active channels'
 // delays: it needs ascending delays (no channel of a group is delayed less than
 // its first) and sums that its narrow lanes hold.
@@ -125,12 +127,15 @@ private:
     struct Setup;
     void prepare(const TddView& v, const TddCall& c);
     void choose_form(const TddView& v, const TddCall& c);
+    void choose_gulp(const TddView& v, const TddCall& c, bool shared);
+    TddHostCall host_call(const TddView& v, const TddCall& c, bool shared, size_t gulp) const;
     void size_rows(const TddView& v, int nbits);
     // Gives back the tables that the current form does not use; true if there
     // were any.
     bool drop_idle_tables();
 
     GpuState& m_gpu;
+    bool m_pinned = false;  // the current call's host buffers: copies overlap on them
     std::unique_ptr<Setup> m_setup;
     rt::DeviceBuffer m_chan, m_cdl, m_km, m_dms, m_perm, m_tr, m_q, m_out[2], m_stage[2];
     PatternTables m_tables[3];  // 16, 8, 4 words per lane

@@ -30,6 +30,15 @@
 
 namespace dedisp {
 namespace kern {
+
+int tdd_sm_count()
+{
+    int dev = 0, sms = 0;
+    RT_CHECK(cudaGetDevice(&dev));
+    RT_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return sms;
+}
+
 namespace {
 
 constexpr int G = kPatternGroup;    // channels per group
@@ -792,21 +801,13 @@ void launch_shape(const DedisperseArgs& a, cudaStream_t s)
     RT_CHECK(cudaGetLastError());
 }
 
-int sm_count()
-{
-    int dev = 0, sms = 0;
-    RT_CHECK(cudaGetDevice(&dev));
-    RT_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    return sms;
-}
-
 template <int MODE, int J>
 void launch_batch_shape(const BatchLaunch& b, cudaStream_t s)
 {
     auto kfn = dedisperse_pattern_batch_kernel<MODE, J>;
     rt::raise_smem_limit(kfn, kDynBytes);
     const unsigned grid =
-        (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(sm_count(), b.total_items));
+        (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(tdd_sm_count(), b.total_items));
     kfn<<<grid, Warps<MODE, J>::NT, kDynBytes, s>>>(b.args, b.item_start, b.nbx, b.nbeams, wait_cfg());
     RT_CHECK(cudaGetLastError());
 }
@@ -849,7 +850,7 @@ int build_warps(int lane_words)
 // trials x 95572 samples, 36 and 72 waves (8 bits 33.2 and 35.8 ms).
 int pattern_lane_words(int nbits, size_t tiles_at_4, long group_words)
 {
-    const size_t sms = (size_t)sm_count();
+    const size_t sms = (size_t)tdd_sm_count();
     const int c = mode_of(nbits) == kBytes ? 6 : 1;
     int best = 0;
     size_t least = 0;

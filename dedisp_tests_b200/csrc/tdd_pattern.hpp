@@ -63,6 +63,8 @@ struct PatternTableArgs {
 void launch_pattern_sizes(const PatternTableArgs& a, cudaStream_t s);
 void launch_pattern_tables(const PatternTableArgs& a, unsigned pieces, cudaStream_t s);
 
+int tdd_sm_count();  // of the current device
+
 // Words per lane (period P = 32 x that) for a call of `tiles_at_4` blocks at 4
 // words per lane, whose widest group stages group_words words beyond the
 // periods of its 8 rows; 0 if none fits.
