@@ -1413,6 +1413,7 @@ __global__ void __launch_bounds__(MAC_THREADS) mac_plain_kernel(MacArgs a, int b
 constexpr int TAB_THREADS = 256;
 constexpr int TAB_CK = 128;      // channels staged at a time
 constexpr int TAB_MAX_TS = 10;
+constexpr int TAB_ENTRIES = 40;  // table entries a thread builds, where there are threads
 constexpr int TAB_MIRROR_TS = 4;  // segment tiles up to this take mirrored bins
 
 __device__ __forceinline__ float2 lds_float2(uint32_t addr)
@@ -1423,7 +1424,7 @@ __device__ __forceinline__ float2 lds_float2(uint32_t addr)
 }
 
 template <int TS, int TM, bool MIRROR>
-__global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel(MacArgs a, int dmax, int bins_per_block, int ts, int groups)
+__global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel(MacArgs a, int dmax, int bins_per_block, int ts, int ndt, int groups)
 {
     extern __shared__ __align__(16) float2 s_tab[];
     const unsigned tab_n = ((unsigned)dmax + 2u) & ~1u;  // even counts keep the arrays aligned
@@ -1436,8 +1437,10 @@ __global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel
     float2* xs = hi + ((nhi + 1u) & ~1u);                       // [TAB_CK][width]
     float* dl = reinterpret_cast<float*>(xs + TAB_CK * width);  // [TAB_CK]
     const int tid = threadIdx.x, nt = blockDim.x;
-    // thread = (segment group, DM thread); whole warps share a group
-    const int ndt = nt / groups, group = tid / ndt, dt = tid - group * ndt;
+    // thread = (segment group, DM thread); whole warps share a group, and those
+    // past the last group only build the table and stage channels
+    const int group = tid / ndt, dt = tid - group * ndt;
+    const bool sums = group < groups;
     for (unsigned i = tid; i < 256; i += nt) lo[i] = a.tw.lo[i];
     for (unsigned i = tid; i < nhi; i += nt) hi[i] = a.tw.hi[i];
     const bool rn = a.round_delays != 0;
@@ -1488,7 +1491,7 @@ __global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel
                     __syncthreads();
                     const float2* xc = xs + group * TS;
 #pragma unroll 2
-                    for (int c = 0; c < nc; ++c, xc += width) {
+                    for (int c = 0; sums && c < nc; ++c, xc += width) {
                         const float delay = dl[c];
                         float2 av[SIDES][TM];
 #pragma unroll
@@ -1526,7 +1529,7 @@ __global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel
 #pragma unroll
                 for (int q = 0; q < TM; ++q) {
                     const int m = m0 + dt + q * ndt;
-                    if (m >= a.ndm) continue;
+                    if (!sums || m >= a.ndm) continue;
 #pragma unroll
                     for (int s = 0; s < TS; ++s)
 #pragma unroll
@@ -1854,15 +1857,15 @@ void launch_fdd_spectrum_out(const float2* Yt, size_t ndm, size_t nspec, float* 
 }
 
 namespace {
-// Threads over DMs first; where those are too few to build the table (40
-// entries a thread) groups of threads take segments of their own.
+// Threads over DMs first; where those are too few to build the table (TAB_ENTRIES
+// a thread) groups of threads take segments of their own.
 struct TableShape {
     int tm, ndt, ts, groups;
     TableShape(int ndm, int nseg, int dmax)
     {
         tm = nseg == 1 && ndm > 4 * TAB_THREADS ? 8 : ndm >= 128 ? 4 : ndm >= 64 ? 2 : 1;
         ndt = std::min(TAB_THREADS, ((ndm + tm - 1) / tm + 31) / 32 * 32);
-        const int most = std::max(1, std::min(TAB_THREADS, dmax / 40) / ndt);
+        const int most = std::max(1, std::min(TAB_THREADS, dmax / TAB_ENTRIES) / ndt);
         const int passes = (nseg + TAB_MAX_TS * most - 1) / (TAB_MAX_TS * most);
         ts = (nseg + passes * most - 1) / (passes * most);
         groups = std::min(most, (nseg + ts - 1) / ts);
@@ -1873,10 +1876,27 @@ struct TableShape {
 bool fdd_mac_table_fits(int dmax, unsigned nfft, int ndm, int nact, int nseg)
 {
     if (dmax < 0 || dmax >= (1 << 22) || nfft % 256 != 0 || nseg < 1 || ndm < 1) return false;
-    // more table entries than phasors used: with enough segments for its tile
-    // the tiled kernel is the faster one (64 DMs x 256 channels x 49 segments,
-    // 18347 delays: 5.3 ms against 7.5)
-    if (nseg > TAB_MAX_TS && (long)dmax > (long)ndm * nact) return false;
+    // The tiled kernel computes 64 phasors per channel and started block of 64 DMs,
+    // for 8 or, above 8 segments, 40 of them at once; the table has dmax entries
+    // whatever the DMs. Table against tiled kernel over 1728 shapes (transforms of
+    // 4096 to 16384 points, 1 to 256 DMs, 32 to 256 channels, delays of 0.1 to
+    // 0.9 of the transform), by entries per tiled phasor: 2 to 4 segments 0.61 to
+    // 0.94 of its time at 1 to 1.5, 0.94 to 1.22 at 2 to 2.5; 5 to 8 segments up to
+    // 1.0 at 0.3 to 0.4, 1.18 at 0.6, 1.32 at 2; 9 and 10 segments 0.73 at 2, 1.1
+    // at 3.6, 1.7 at 7. Above 10 the tiles are well filled and the entries count
+    // against the DMs there are: at 0.9 0.43 to 0.93, but 64 DMs x 256 channels x
+    // 14745 delays 0.94 to 1.15 (a table of one block an SM, two DMs a thread); 64
+    // x 256 x 49 segments x 18347 delays 7.5 ms against 5.3. One segment always
+    // takes the table: phasors from the twiddle tables for single products are
+    // what it replaced.
+    const double tiled = (double)((ndm + 63) / 64 * 64) * nact;
+    const bool lean = ndm < 128 && dmax > 10000;
+    if (nseg > TAB_MAX_TS ? dmax > (lean ? 0.85 : 1.0) * (double)ndm * nact
+        : nseg > 8        ? dmax > 3.0 * tiled
+        : nseg > 4        ? dmax > 0.5 * tiled
+        : nseg > 1        ? dmax > 1.75 * tiled
+                          : false)
+        return false;
     const TableShape t(ndm, nseg, dmax);
     // 200 KB for the tables of one segment (lengths up to 6.4 million samples
     // at small delays, more than the tiled kernel takes) and its staged columns
@@ -1891,11 +1911,12 @@ void launch_mac_table(const MacArgs& a, int dmax, int ts, int ndt, int groups, c
     auto kfn = mac_table_kernel<TS, TM, MIRROR>;
     const size_t smem = table_smem_bytes(dmax, a.nfft, (MIRROR ? 2 : 1) * TS * groups);
     rt::raise_smem_limit(kfn, smem);
-    const unsigned nt = (unsigned)(ndt * groups);
+    // few DMs and segments leave too few threads for a long table
+    const unsigned nt = (unsigned)std::max(ndt * groups, std::min(TAB_THREADS, dmax / TAB_ENTRIES / 32 * 32));
     const size_t units = MIRROR ? (size_t)a.nfft / 4 + 1 : a.nbins;
     const unsigned grid = persistent_grid(kfn, nt, smem, units);
     const int per = (int)((units + grid - 1) / grid);
-    kfn<<<(unsigned)((units + per - 1) / per), nt, smem, s>>>(a, dmax, per, ts, groups);
+    kfn<<<(unsigned)((units + per - 1) / per), nt, smem, s>>>(a, dmax, per, ts, ndt, groups);
     RT_CHECK(cudaGetLastError());
 }
 
