@@ -1370,12 +1370,14 @@ __global__ void __launch_bounds__(MAC_THREADS) mac_plain_kernel(MacArgs a, int b
     }
 }
 
-// FP32 MAC with a phasor table per bin: the form that runs whenever every delay
-// index 0..dmax fits shared memory. Per bin the CTA builds the phasors of all
+// FP32 MAC with a phasor table per bin, where every delay index 0..dmax fits
+// shared memory and the table is worth building (fdd_mac_table_fits). Per bin the CTA builds the phasors of all
 // delays (index k d mod N stepped exactly by (k nt) mod N, the same phasor()
 // product as the tiled kernel), then each thread accumulates TM DMs x TS
 // segments over all channels, in the tiled kernel's channel order and FMA
-// sequence, so the sums are the same bit for bit. A phasor costs a delay (dm *
+// sequence: the same sums bit for bit, but for the upper half of the bins in
+// tiles that take mirrored ones (below), whose phasors are rounded at the bin
+// they mirror. A phasor costs a delay (dm *
 // delay rounded by adding 2^23, toward zero or to nearest even: exact for 0 <=
 // dm * delay < 2^22, which dmax bounds) and one shared load that neighbouring
 // DMs take from neighbouring entries, and feeds 2 TS packed FMAs; the channel's

@@ -122,8 +122,10 @@ struct MacArgs {
     TwiddleTable tw;
 };
 void launch_fdd_mac_plain(const MacArgs& a, cudaStream_t s);
-// The same sums with a per-bin phasor table over delays 0..dmax (the largest
-// delay index of the plan's DMs and channels). No DM and no delay may be
+// The same products with a per-bin phasor table over delays 0..dmax (the largest
+// delay index of the plan's DMs and channels), in the same order; in tiles of up
+// to four segments the phasors of bins above N/4 are those of N/2 - k mirrored,
+// which differ in their last bits. No DM and no delay may be
 // negative or NaN: the kernel reads the table without a check of the index.
 // fdd_mac_table_fits: dmax known, the tables fit, and building them is not the
 // larger part of the work.
