@@ -36,7 +36,8 @@ bool pattern_takes(const std::vector<float>& dms, const std::vector<float>& dela
     if (nbits == 16 && nact > 65536u) return false;                       // 32-bit sums
     if (!(delays.front() >= 0.f) || !std::is_sorted(delays.begin(), delays.end())) return false;
     if ((dms.size() + kern::kPatternDms - 1) / kern::kPatternDms > 65535) return false;
-    return hostmath::delay_rn(dms.back(), delays.back()) < (1u << 30);
+    // (the tables add up 8 rows and 32 series of the delays' span in 32 bits)
+    return hostmath::delay_rn(dms.back(), delays.back()) < (1u << 25);
 }
 
 // Everything derived from (DM list, killmask, DM range, nbits, kernel choice).

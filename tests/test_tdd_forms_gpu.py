@@ -125,3 +125,35 @@ def test_batch_form(nbits, nouts, lane_words):
             assert same(np.ascontiguousarray(a[:, :nout]), oracle(packed, nbits, dms, nout))
             assert np.all(a[:, nout:] == -7.0)
     b.close()
+
+
+def test_delays_past_the_tables_sums():
+    """Delays of 2^25 samples and more: the tables' sizes would pass 32 bits, so
+    such lists run row by row (or plain) without asking for them."""
+    import torch
+    nch, nout = 32, 300
+    params = (nch, 1e-6, 400.0, -1.0)
+    p = dd.TDDPlan(*params)
+    p.set_dm_list(np.array([1000.0], np.float32))
+    dm = 1000.0 * 2.0 ** 25.1 / p.get_max_delay()
+    dms = np.linspace(dm * (1 - 1e-6), dm, 40).astype(np.float32)
+    p.set_dm_list(dms)
+    md = p.get_max_delay()
+    assert md > 1 << 25
+    n = nout + md
+    x = torch.randint(0, 2, (n, nch), dtype=torch.uint8, device="cuda")
+    words = (x.to(torch.int32) << torch.arange(nch, device="cuda", dtype=torch.int32)).sum(1, dtype=torch.int64)
+    packed = (words & 0xFFFFFFFF).to(torch.uint32).view(torch.uint8)
+    out = torch.zeros((len(dms), nout), dtype=torch.float32, device="cuda")
+    for _ in range(2):
+        p.execute(n, packed, 1, out, 32, dd.DEDISP_DEVICE_POINTERS)
+        assert p.get_form()[0] in ("rows", "plain")
+    delays = po.delay_table(nch, *[np.float32(v) for v in params[1:]])
+    got = out.cpu().numpy()
+    xs = x.cpu().numpy()
+    scale = np.float32(3.0 * 1024.0 / 255.0 / 16.0)
+    for i in (0, 17, 39):
+        d = np.rint((dms[i] * delays[:nch]).astype(np.float32)).astype(np.int64)
+        want = sum(xs[k:k + nout, c].astype(np.float32) for c, k in enumerate(d))
+        want = (want / np.float32(nch)).astype(np.float32) * scale
+        assert np.array_equal(got[i], want), i
