@@ -1017,16 +1017,39 @@ def run_ours(args):
                         f"({tiles_cap} tiles), scaled to this launch's {tiles} tiles; not measured "
                         f"in this run")
     achieved = adds / (k2_ms * 1e-3) / 1e12
-    roofline = {"bound": "int-alu", "achieved": round(achieved, 3), "peak": round(peak.value / 1e12, 3),
-                "unit": "Tadd/s", "frac": round(achieved * 1e12 / peak.value, 4),
+    alu = {"bound": "int-alu", "achieved": round(achieved, 3), "peak": round(peak.value / 1e12, 3),
+           "unit": "Tadd/s", "frac": round(achieved * 1e12 / peak.value, 4),
+           "peak_source": "measured in this run: dedisp_probe_alu (lib/libdedisp_probe.so; 32-bit add "
+                          "lane-ops/s, all SMs)"}
+    form = plan.get_form()
+    if form[0] == "shared":
+        # Trials share the sums of channel groups, so one add per channel and
+        # sample bounds nothing: shared-memory wavefronts do, one per SM and
+        # clock. Counted in the same capture, 6.93e9 over 47 tiles at 16 words
+        # per lane; they are a property of the DM list and the tiles.
+        waves = None
+        if traffic is not None and form[1] == 16:
+            waves = 6.93e9 / 47 * -(-nout // 2048)
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
+        top = sms * (clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 0) * 1e6
+        got = waves / (k2_ms * 1e-3) if waves else None
+        bound = {"bound": "shared-memory wavefronts", "unit": "Gwavefront/s",
+                 "achieved": round(got / 1e9, 2) if got else None,
+                 "peak": round(top / 1e9, 2) if top else None,
+                 "frac": round(got / top, 4) if got and top else None,
+                 "peak_source": "one wavefront per SM and clock, SM clock sampled in this run; wavefronts "
+                                "from the ncu capture of the workload cut to 2^17 samples, scaled to this "
+                                "launch's tiles",
+                 "adds_view": {k: alu[k] for k in ("achieved", "peak", "unit", "peak_source")}}
+    else:
+        bound = alu
+    roofline = {**bound,
                 "traffic": traffic,
                 "traffic_source": traffic_note,
-                "peak_source": "measured in this run: dedisp_probe_alu (lib/libdedisp_probe.so; 32-bit add "
-                               "lane-ops/s, all SMs)",
                 "k2_ms": round(k2_ms, 3), "k1_ms": round(sum(pms) / len(pms), 3),
-                "algorithmic": "nchan=4096 integer adds per DM-trial x sample (variant 5 shares sums of "
-                               "channel groups between trials and so needs fewer: frac may pass 1); "
-                               f"{adds:.3e} adds per step",
+                "kernel_form": {"name": form[0], "lane_words": form[1], "rounds": form[2]},
+                "algorithmic": "nchan=4096 integer adds per DM-trial x sample, fewer where trials share sums "
+                               f"of channel groups; {adds:.3e} adds per step",
                 "hbm_view": {"algorithmic_bytes": int(cfg.nsamps * 4096 * args.nbits // 8 +
                                                       units * 4),
                              "achieved_GBs": round((cfg.nsamps * 4096 * args.nbits // 8 +
@@ -1065,10 +1088,12 @@ def run_ours(args):
             torch.cuda.synchronize()
             vm = max_over_ranks(ev0.elapsed_time(ev1)) / 2
             t = p2.get_timing()
+            # (no fraction of a bound where sums are shared: may pass 1)
             variants[f"tiled_{nb}bit"] = {"value": units * world / (vm * 1e-3),
                                           "ms_per_step": vm, "kernel_ms": t["kernel_ms"],
-                                          "frac_int_alu": round(adds / (t["kernel_ms"] * 1e-3)
-                                                                / peak.value, 4)}
+                                          "kernel_form": p2.get_form()[0],
+                                          "adds_over_int_alu_peak": round(adds / (t["kernel_ms"] * 1e-3)
+                                                                          / peak.value, 4)}
             del inp, p2
         variants[f"tiled_{args.nbits}bit"] = {"value": value, "ms_per_step": ms,
                                               "kernel_ms": k2_ms}
