@@ -461,13 +461,8 @@ __device__ __forceinline__ void pattern_stage(const DedisperseArgs& a, size_t t0
         if (p + 2 < pieces && lane <= G) next[1] = __ldg(win + (size_t)(p + 2) * 16 + lane);
         const int after = (int)__shfl_sync(FULL, c.y, 0);
         const uint32_t slot = __shfl_sync(FULL, c.w, 0);
-        // (the warp leaves as one: a lane that went on alone would wait for the
-        // others in the next shuffle for good)
-        const bool ok = after < 0 || piece_wait(y.summed, after, wc.ns);
-        if (!__all_sync(FULL, ok)) {
-            if (lane == 0) atomicExch(&y.failed, 1);
-            return;
-        }
+        // addresses before the wait: what follows it is on the chain from one
+        // piece's sums to the next piece's rows
         uint64_t* full = &y.full[p & (LIVE - 1)];
         uint32_t n = c.z;
         const uint32_t* src = a.rec + (size_t)c.x * a.rec_stride;
@@ -478,6 +473,12 @@ __device__ __forceinline__ void pattern_stage(const DedisperseArgs& a, size_t t0
             const size_t room = a.tr_pitch_words > first ? a.tr_pitch_words - first : 0;
             if (room < n) n = (uint32_t)room;
             src = a.tr + (size_t)c.x * a.tr_pitch_words + first;
+        }
+        // (the warp leaves as one: a lane that went on alone would wait for the
+        // others in the next shuffle for good)
+        if (after >= 0 && !__all_sync(FULL, piece_wait(y.summed, after, wc.ns))) {
+            if (lane == 0) atomicExch(&y.failed, 1);
+            return;
         }
         if (lane <= G && n) {
             mbar_expect_tx(full, 4u * n);
