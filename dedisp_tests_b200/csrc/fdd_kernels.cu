@@ -1425,8 +1425,11 @@ __device__ __forceinline__ float2 lds_float2(uint32_t addr)
     return v;
 }
 
-template <int TS, int TM, bool MIRROR>
-__global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel(MacArgs a, int dmax, int bins_per_block, int ts, int ndt, int groups)
+// HELPERS: threads past the DMs and segments' own only build the table and stage
+// channels (a form of its own: the test costs 1.5% at one segment).
+template <int TS, int TM, bool MIRROR, bool HELPERS>
+__global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0)
+mac_table_kernel(MacArgs a, int dmax, int bins_per_block, int ts, int own_ndt, int groups)
 {
     extern __shared__ __align__(16) float2 s_tab[];
     const unsigned tab_n = ((unsigned)dmax + 2u) & ~1u;  // even counts keep the arrays aligned
@@ -1439,10 +1442,9 @@ __global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel
     float2* xs = hi + ((nhi + 1u) & ~1u);                       // [TAB_CK][width]
     float* dl = reinterpret_cast<float*>(xs + TAB_CK * width);  // [TAB_CK]
     const int tid = threadIdx.x, nt = blockDim.x;
-    // thread = (segment group, DM thread); whole warps share a group, and those
-    // past the last group only build the table and stage channels
-    const int group = tid / ndt, dt = tid - group * ndt;
-    const bool sums = group < groups;
+    // thread = (segment group, DM thread); whole warps share a group
+    const int ndt = HELPERS ? own_ndt : nt / groups, group = tid / ndt, dt = tid - group * ndt;
+    const bool helper = HELPERS && group >= groups;
     for (unsigned i = tid; i < 256; i += nt) lo[i] = a.tw.lo[i];
     for (unsigned i = tid; i < nhi; i += nt) hi[i] = a.tw.hi[i];
     const bool rn = a.round_delays != 0;
@@ -1491,9 +1493,10 @@ __global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel
                     }
                     for (int i = tid; i < nc; i += nt) dl[i] = a.delay_act[c0 + i];
                     __syncthreads();
+                    if (helper) continue;
                     const float2* xc = xs + group * TS;
 #pragma unroll 2
-                    for (int c = 0; sums && c < nc; ++c, xc += width) {
+                    for (int c = 0; c < nc; ++c, xc += width) {
                         const float delay = dl[c];
                         float2 av[SIDES][TM];
 #pragma unroll
@@ -1531,7 +1534,7 @@ __global__ void __launch_bounds__(TAB_THREADS, TS == 1 ? 2 : 0) mac_table_kernel
 #pragma unroll
                 for (int q = 0; q < TM; ++q) {
                     const int m = m0 + dt + q * ndt;
-                    if (!sums || m >= a.ndm) continue;
+                    if (helper || m >= a.ndm) continue;
 #pragma unroll
                     for (int s = 0; s < TS; ++s)
 #pragma unroll
@@ -1906,20 +1909,28 @@ bool fdd_mac_table_fits(int dmax, unsigned nfft, int ndm, int nact, int nseg)
 }
 
 namespace {
-template <int TS, int TM>
-void launch_mac_table(const MacArgs& a, int dmax, int ts, int ndt, int groups, cudaStream_t s)
+template <int TS, int TM, bool HELPERS>
+void launch_mac_table_form(const MacArgs& a, int dmax, unsigned nt, int ts, int ndt, int groups, cudaStream_t s)
 {
     constexpr bool MIRROR = TS <= TAB_MIRROR_TS;
-    auto kfn = mac_table_kernel<TS, TM, MIRROR>;
+    auto kfn = mac_table_kernel<TS, TM, MIRROR, HELPERS>;
     const size_t smem = table_smem_bytes(dmax, a.nfft, (MIRROR ? 2 : 1) * TS * groups);
     rt::raise_smem_limit(kfn, smem);
-    // few DMs and segments leave too few threads for a long table
-    const unsigned nt = (unsigned)std::max(ndt * groups, std::min(TAB_THREADS, dmax / TAB_ENTRIES / 32 * 32));
     const size_t units = MIRROR ? (size_t)a.nfft / 4 + 1 : a.nbins;
     const unsigned grid = persistent_grid(kfn, nt, smem, units);
     const int per = (int)((units + grid - 1) / grid);
     kfn<<<(unsigned)((units + per - 1) / per), nt, smem, s>>>(a, dmax, per, ts, ndt, groups);
     RT_CHECK(cudaGetLastError());
+}
+
+template <int TS, int TM>
+void launch_mac_table(const MacArgs& a, int dmax, int ts, int ndt, int groups, cudaStream_t s)
+{
+    // few DMs and segments leave too few threads for a long table
+    const int own = ndt * groups, nt = std::min(TAB_THREADS, dmax / TAB_ENTRIES / 32 * 32);
+    if constexpr (TM < 8)
+        if (nt > own) return launch_mac_table_form<TS, TM, true>(a, dmax, (unsigned)nt, ts, ndt, groups, s);
+    launch_mac_table_form<TS, TM, false>(a, dmax, (unsigned)own, ts, ndt, groups, s);
 }
 
 template <int TS>
