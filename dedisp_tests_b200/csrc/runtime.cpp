@@ -7,6 +7,7 @@
 #include <map>
 #include <mutex>
 #include <sstream>
+#include <vector>
 
 namespace dedisp {
 
@@ -115,6 +116,50 @@ void PinnedBuffer::release()
     if (m_ptr) cudaFreeHost(m_ptr);
     m_ptr = nullptr;
     m_cap = 0;
+}
+
+namespace {
+struct PinnedPage {
+    std::mutex m;
+    PinnedBuffer page;
+    std::vector<unsigned*> spare;
+    bool tried = false;
+};
+// (never destroyed: the CUDA runtime may be gone by then)
+PinnedPage& pinned_page()
+{
+    static PinnedPage* p = new PinnedPage;
+    return *p;
+}
+}  // namespace
+
+unsigned* PinnedWord::get()
+{
+    if (m_ptr) return m_ptr;
+    PinnedPage& p = pinned_page();
+    std::lock_guard<std::mutex> lk(p.m);
+    if (!p.tried) {
+        p.tried = true;
+        try {
+            p.page.reserve(4096);
+            for (size_t i = 4096 / sizeof(unsigned); i-- > 0;) p.spare.push_back(p.page.get<unsigned>() + i);
+        } catch (const Error&) {
+            cudaGetLastError();  // callers do without
+        }
+    }
+    if (p.spare.empty()) return nullptr;
+    m_ptr = p.spare.back();
+    p.spare.pop_back();
+    return m_ptr;
+}
+
+void PinnedWord::release()
+{
+    if (!m_ptr) return;
+    PinnedPage& p = pinned_page();
+    std::lock_guard<std::mutex> lk(p.m);
+    p.spare.push_back(m_ptr);
+    m_ptr = nullptr;
 }
 
 Stream::Stream() { RT_CHECK(cudaStreamCreateWithFlags(&m_s, cudaStreamNonBlocking)); }

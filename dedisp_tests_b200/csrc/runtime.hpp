@@ -78,6 +78,22 @@ private:
     size_t m_cap = 0;
 };
 
+// A word of pinned host memory for a kernel's status, from one page that the
+// process allocates at the first use (an allocation per plan cost each plan's
+// first call 2 to 9 ms). 1024 at a time; get() is null for more.
+class PinnedWord {
+public:
+    PinnedWord() = default;
+    ~PinnedWord() { release(); }
+    PinnedWord(const PinnedWord&) = delete;
+    PinnedWord& operator=(const PinnedWord&) = delete;
+    unsigned* get();  // takes a word at the first call
+    void release();
+
+private:
+    unsigned* m_ptr = nullptr;
+};
+
 class Stream {
 public:
     Stream();

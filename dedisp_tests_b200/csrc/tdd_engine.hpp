@@ -139,6 +139,7 @@ private:
     std::unique_ptr<Setup> m_setup;
     rt::DeviceBuffer m_chan, m_cdl, m_km, m_dms, m_perm, m_tr, m_q, m_out[2], m_stage[2];
     PatternTables m_tables[3];  // 16, 8, 4 words per lane
+    rt::PinnedWord m_err_host;
     rt::DeviceBuffer m_err;  // set by a quad-strided kernel whose bounded wait expired
     std::vector<std::unique_ptr<rt::Event>> m_events;
     rt::Event& event(size_t i);

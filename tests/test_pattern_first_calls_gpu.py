@@ -86,3 +86,27 @@ def test_captured_call_outlives_the_change_of_form(warm):
     assert same(y.cpu().numpy(), want)
     del g
     p.set_stream(0)
+
+
+def test_more_plans_than_status_words():
+    """Plans take a status word each from one page of 1024; those past it, and
+    those that take a word given back, give the same results."""
+    dms, nout = fine_list(8), 300
+    packed = series(8, nout + plan(dms).get_max_delay(), 9)
+    want = oracle(packed, 8, dms, nout)
+
+    def run(p):
+        out = np.zeros((len(dms), nout), np.float32)
+        p.execute(packed.shape[0], packed, 8, out, 32)
+        assert same(out, want)
+
+    plans = [plan(dms) for _ in range(1030)]
+    for p in plans:
+        run(p)
+    for p in plans[1000:]:
+        run(p)
+    for p in plans[:20]:
+        p.close()
+    run(plan(dms))
+    for p in plans[20:]:
+        p.close()
