@@ -33,7 +33,9 @@ dedisp_error dedisp_b200_set_tdd_kernel(dedisp_plan plan, int kernel);
  * the executed width's range selects that width's default (quad-strided
  * 20 words x 12 DMs for widths up to 8 bits). The default variant, set or not,
  * runs the kernel on shared channel-group sums (csrc/tdd_pattern.hpp) where that
- * is the faster one for the DM list. Every variant computes the same
+ * is the faster one for the DM list; a small call (below 2e9 additions) on a new
+ * list, mask, DM range or width runs row by row and leaves its tables to the
+ * next. Every variant computes the same
  * bit-exact sums; they differ in speed. */
 dedisp_error dedisp_b200_set_tdd_variant(dedisp_plan plan, int variant);
 int dedisp_b200_tdd_variant_count(dedisp_size in_nbits);
@@ -104,8 +106,8 @@ dedisp_error dedisp_b200_set_fdd_options(dedisp_plan plan, int segmented, int ti
                                          dedisp_size segment_nfft);
 
 /* Bounded device waits. No counterpart in the reference (its kernels do not
- * wait on asynchronous copies). The quad-strided TDD kernels and the
- * tensor-core FDD MAC poll mbarriers for their own bulk copies and MMAs; a
+ * wait on asynchronous copies). The quad-strided and shared-sum TDD kernels and
+ * the tensor-core FDD MAC poll mbarriers for their own bulk copies and MMAs; a
  * poll that has not seen its phase complete after `ns` nanoseconds of GPU
  * global time gives up: the kernel waits (bounded again) for its own work
  * still in flight, frees its tensor memory and returns, and the plan's
@@ -135,7 +137,9 @@ dedisp_error dedisp_b200_set_wait_expiry_test(int enable);
  * library (plus small tables for up to 16384 DMs and 8192 channels), held by
  * every GPU that loads the library until the process exits. Requests whose
  * channel-major copy, (nchans + 1) x (nsamps rounded up + padding) samples,
- * does not fit are rejected with DEDISP_MEM_ALLOC_FAILED. The first call on
+ * does not fit are rejected with DEDISP_MEM_ALLOC_FAILED. It runs the
+ * row-by-row kernel on packed rows: the shared channel-group sums that plans
+ * take need tables and larger rows than the scratch holds. The first call on
  * a device looks up the arrays' device addresses (cudaGetSymbolAddress) and
  * should therefore come before any stream capture on that device; `stream`
  * (NULL: the legacy default stream) must belong to the current device
