@@ -91,6 +91,7 @@ TddBatch::TddBatch(size_t nchans, float dt, float f0, float df, int in_nbits, in
     set_killmask(nullptr);
     rt::DeviceGuard g(m_device);
     for (auto& e : m_ev) e.reset(new rt::Event(true));
+    m_done.reset(new rt::Event(false));
     m_d_delay.reserve(m_delays.size() * 4);
     m_d_err.reserve(sizeof(unsigned));
     RT_CHECK(cudaMemset(m_d_err.get(), 0, sizeof(unsigned)));
@@ -103,6 +104,13 @@ TddBatch::~TddBatch()
     if (cudaGetDevice(&cur) == cudaSuccess && cur != m_device) cudaSetDevice(m_device);
     cudaDeviceSynchronize();
     drop_graph();
+}
+
+void TddBatch::wait_in_flight()
+{
+    if (!m_in_flight) return;
+    m_in_flight = false;
+    RT_CHECK(cudaEventSynchronize(*m_done));
 }
 
 void TddBatch::drop_graph()
@@ -134,6 +142,7 @@ void TddBatch::set_killmask(const int32_t* killmask)
     std::vector<float> cdl(padded.size());  // delay of each list entry
     for (size_t j = 0; j < padded.size(); ++j) cdl[j] = m_delays[padded[j]];
     rt::DeviceGuard g(m_device);
+    wait_in_flight();
     m_d_chan.reserve(padded.size() * 4);
     RT_CHECK(cudaMemcpy(m_d_chan.get(), padded.data(), padded.size() * 4, cudaMemcpyHostToDevice));
     m_d_cdl.reserve(cdl.size() * 4);
@@ -186,6 +195,7 @@ void TddBatch::set_beams(std::vector<BatchBeamSpec> beams)
         t.spec = std::move(s);
     }
     rt::DeviceGuard g(m_device);
+    wait_in_flight();
     std::vector<float> dms(std::max<size_t>(dm_total, 1), 0.f);
     std::vector<int32_t> perm(std::max<size_t>(dm_total, 1), 0);
     for (auto& t : st) {
@@ -427,6 +437,7 @@ uint8_t* TddBatch::workspace_base()
 void TddBatch::upload(Layout& L)
 {
     rt::DeviceGuard g(m_device);
+    wait_in_flight();
     uint32_t* ws = reinterpret_cast<uint32_t*>(workspace_base());
     std::vector<kern::DedisperseArgs> args(L.args);
     for (size_t b = 0; b < m_beams.size(); ++b) {
@@ -606,6 +617,12 @@ void TddBatch::execute(cudaStream_t stream, bool use_graph)
         RT_CHECK(cudaGraphLaunch(m_exec, stream));
         if (record_timing) m_ev[2]->record(stream);
         last_launches = m_graph_launches;
+    }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    RT_CHECK(cudaStreamIsCapturing(stream, &cap));
+    if (cap == cudaStreamCaptureStatusNone) {
+        m_done->record(stream);
+        m_in_flight = true;
     }
     if (record_timing) {
         RT_CHECK(cudaEventSynchronize(m_ev[2]->get()));

@@ -93,6 +93,9 @@ private:
     // rows do not fit it, DEDISP_MEM_ALLOC_FAILED where neither does.
     Layout fitting_layout(const BatchShape& shape, size_t tile_limit_samples) const;
     size_t workspace_words(bool shared) const;
+    // Waits for the last execute: its kernels read the device lists and tables
+    // that are about to be written, on a stream that need not wait for ours.
+    void wait_in_flight();
     uint32_t delay_span(const BeamState& t, size_t block_dms) const;
     void upload(Layout& L);
     void prepare_patterns();
@@ -125,6 +128,8 @@ private:
     cudaGraphExec_t m_exec = nullptr;
     int m_graph_launches = 0;     // kernel launches inside the captured graph
     std::unique_ptr<rt::Event> m_ev[3];
+    std::unique_ptr<rt::Event> m_done;  // behind the last execute
+    bool m_in_flight = false;
 };
 
 }  // namespace detail

@@ -157,3 +157,36 @@ def test_delays_past_the_tables_sums():
         want = sum(xs[k:k + nout, c].astype(np.float32) for c, k in enumerate(d))
         want = (want / np.float32(nch)).astype(np.float32) * scale
         assert np.array_equal(got[i], want), i
+
+
+def test_batch_set_again_while_it_runs():
+    """New beams and a new mask right behind an execute on a stream of its own:
+    the lists and tables that its kernels still read are written after it."""
+    import torch
+    s = torch.cuda.Stream()
+    lists, nouts = [fine_list(640, 5.0), fine_list(320)], (40000, 30000)
+    b, ins, outs, beams = make_batch(8, lists, nouts, seed=3)
+    other, nout2 = [fine_list(96, step=0.05)], 5000
+    b2, ins2, outs2, beams2 = make_batch(8, other, [nout2], seed=9)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        for graph in (False, True):
+            for y in outs + outs2:
+                y.zero_()
+            b.set_beams(beams)
+            s.synchronize()
+            b.execute(s.cuda_stream, use_graph=graph)
+            first = b.get_form()[0]
+            b.set_beams(beams2)
+            b.execute(s.cuda_stream, use_graph=graph)
+            km = np.ones(NCH, np.int32)
+            km[::3] = 0
+            b.set_killmask(km)
+            b.set_killmask(None)
+            b.sync(s.cuda_stream)
+            assert first == "shared" and b.get_form()[0] == "shared"
+            for packed, dms, y in zip(ins, lists, outs):
+                assert same(y[:, :2000].contiguous().cpu().numpy(),
+                            np.ascontiguousarray(oracle(packed, 8, dms, 2000)))
+            assert same(outs2[0].cpu().numpy(), oracle(ins2[0], 8, other[0], nout2))
+    b.close()
